@@ -984,44 +984,76 @@ __device__ __forceinline__ uint32_t old_lower_bound(const Queue& q, float d, uin
     return lo;
 }
 
-// Merges the m (<= kCandBatch) accepted entries of bd/bv into the sorted
-// array and trims it at the new lb. The batch is first sorted by (dist, vid)
-// in place (each lane holds at most two entries in registers). A vid word may
-// carry the explored bit (an entry popped before it is merged); ordering
-// ignores it.
-// Returns true when an entry that may still be live was dropped: with a
-// capacity below 2L (the compact layout), entries past the capacity are not
-// kept; they are dead unless every kept entry past L ties lb, which is what
-// is reported (the caller then hands the query to the full-capacity rerun).
-__device__ inline bool queue_merge(Queue& q, float* bd, uint32_t* bv, uint32_t m) {
-    const int lane = lane_id();
-    if (m == 0) return false;
-    const bool truncated = q.n + m > q.cap;
-    {
-        float sd[2];
-        uint32_t sv[2], rk[2];
+// Places the m <= kFew sorted entries of bd/bv into the sorted array q[0, n), n
+// >= 1: an old entry moves up by the number of batch entries before it; lane r
+// finds batch entry r's rank among the old ones from a ballot a chunk and writes
+// it last. Chunks of 32 entries go tail first; a chunk's outputs lie at or after
+// its own first position, so the next chunk is read before they are written.
+// Chunks before the first batch entry are not touched. Entries past the capacity
+// are dropped. Returns the position of the smallest batch entry.
+// Most merges have one to four entries: counting by comparison against that many
+// registers replaces a binary search of 7-10 dependent shared-memory loads and
+// two cross-lane reductions a chunk.
+// (1M x 128, 10,000 queries: queue 100 4.25 -> 4.00 ms, queue 400 13.97 -> 13.20
+// ms, with the ranking by four entries a step in queue_merge.)
+template <int kFew>
+__device__ __forceinline__ uint32_t queue_place_few(const Queue& q, const float* bd, const uint32_t* bv, uint32_t m) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t n = q.n, cap = q.cap;
+    float rd[kFew];
+    uint32_t rv[kFew];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const uint32_t k = lane + 32u * t;
-            rk[t] = 0xffffffffu;
-            if (k < m) {
-                sd[t] = bd[k];
-                sv[t] = bv[k];
-                uint32_t r = 0;
-                for (uint32_t i = 0; i < m; ++i) r += entry_less(bd[i], bv[i], sd[t], sv[t]) ? 1u : 0u;
-                rk[t] = r;
-            }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            if (rk[t] != 0xffffffffu) {
-                bd[rk[t]] = sd[t];
-                bv[rk[t]] = sv[t];
-            }
-        }
-        __syncwarp();
+    for (int r = 0; r < kFew; ++r) {
+        // Past m: after every entry (an entry at distance NaN, which compares
+        // false with all, counts as after the whole batch).
+        rd[r] = static_cast<uint32_t>(r) < m ? bd[r] : INFINITY;
+        rv[r] = static_cast<uint32_t>(r) < m ? (bv[r] & kVidMask) : 0xffffffffu;
     }
+    uint32_t rank = 0;        // lane r: old entries before batch entry r
+    bool found = false;
+    uint32_t cb = (n - 1u) & ~31u;
+    uint2 w = make_uint2(0u, 0u);
+    if (cb + lane < n) w = q.e[cb + lane];
+    #pragma unroll 1
+    for (;;) {
+        const uint32_t idx = cb + lane;
+        const bool in = idx < n;
+        uint2 wn = make_uint2(0u, 0u);
+        if (cb) wn = q.e[cb - 32u + lane];
+        const float wd = ent_d(w);
+        const uint32_t wv = w.x & kVidMask;
+        uint32_t c = 0;       // batch entries before this one
+        uint32_t before = 0;  // lane r: this chunk's entries before batch entry r
+        bool any0 = false;
+#pragma unroll
+        for (int r = 0; r < kFew; ++r) {
+            const bool less = (wd < rd[r]) | ((wd == rd[r]) & (wv < rv[r]));   // this entry is before batch entry r
+            c += less ? 0u : 1u;
+            const uint32_t b = __ballot_sync(kFull, in & less);
+            if (lane == static_cast<uint32_t>(r)) before = b;
+            if (r == 0) any0 = b != 0u;
+        }
+        c = min(c, m);
+        if (!found && before) {
+            rank = cb + __popc(before);
+            found = true;
+        }
+        __syncwarp();   // the next chunk has been read
+        if (in && c && idx + c < cap) q.e[idx + c] = w;
+        if (any0 || cb == 0u) break;
+        cb -= 32u;
+        w = wn;
+    }
+    __syncwarp();
+    if (lane < m && rank + lane < cap) q.e[rank + lane] = make_ent(bd[lane], bv[lane]);
+    __syncwarp();
+    return __shfl_sync(kFull, rank, 0);
+}
+
+// The same for any m <= kCandBatch: batch entries find their positions by binary
+// search, every output gathers its source.
+__device__ __forceinline__ int queue_place_many(const Queue& q, const float* bd, const uint32_t* bv, uint32_t m) {
+    const int lane = lane_id();
     // Final positions of the batch entries: rank in the old array + rank in
     // the batch (sorted, distinct); lanes past m hold a sentinel above every
     // position.
@@ -1039,6 +1071,7 @@ __device__ inline bool queue_merge(Queue& q, float* bd, uint32_t* bv, uint32_t m
     // before the outputs of every chunk written earlier.
     const int end = static_cast<int>(min(q.n + m, q.cap));
     const uint32_t lt = (1u << lane) - 1u;
+    #pragma unroll 1
     for (int cb = end - 32; cb + 32 > p0; cb -= 32) {
         const uint32_t rel0 = static_cast<uint32_t>(posb0) - static_cast<uint32_t>(cb);
         const uint32_t rel1 = static_cast<uint32_t>(posb1) - static_cast<uint32_t>(cb);
@@ -1058,12 +1091,71 @@ __device__ inline bool queue_merge(Queue& q, float* bd, uint32_t* bv, uint32_t m
         if (act) q.e[o] = ww;
     }
     __syncwarp();
+    return p0;
+}
+
+// Merges the m (<= kCandBatch) accepted entries of bd/bv into the sorted
+// array and trims it at the new lb. The batch is first sorted by (dist, vid)
+// in place (each lane holds at most two entries in registers). A vid word may
+// carry the explored bit (an entry popped before it is merged); ordering
+// ignores it.
+// Returns true when an entry that may still be live was dropped: with a
+// capacity below 2L (the compact layout), entries past the capacity are not
+// kept; they are dead unless every kept entry past L ties lb, which is what
+// is reported (the caller then hands the query to the full-capacity rerun).
+__device__ inline bool queue_merge(Queue& q, float* bd, uint32_t* bv, uint32_t m) {
+    const int lane = lane_id();
+    if (m == 0) return false;
+    const bool truncated = q.n + m > q.cap;
+    if (m > 1u) {
+        // Each lane ranks at most two of the entries, four at a time against
+        // all (entries past m: a sentinel above every one).
+        const uint32_t pad = m + static_cast<uint32_t>(lane);
+        if (lane < 4 && pad < kCandBatch) {
+            bd[pad] = INFINITY;
+            bv[pad] = 0xffffffffu;
+        }
+        __syncwarp();
+        const bool h0 = static_cast<uint32_t>(lane) < m, h1 = static_cast<uint32_t>(lane) + 32u < m;
+        const float d0 = bd[lane], d1 = bd[lane + 32];
+        const uint32_t w0 = bv[lane], w1 = bv[lane + 32];
+        uint32_t r0 = 0, r1 = 0;
+        #pragma unroll 1
+        for (uint32_t i = 0; i < m; i += 4) {
+            const float4 bd4 = *reinterpret_cast<const float4*>(bd + i);
+            const uint4 bv4 = *reinterpret_cast<const uint4*>(bv + i);
+            r0 += entry_less(bd4.x, bv4.x, d0, w0) + entry_less(bd4.y, bv4.y, d0, w0) +
+                  entry_less(bd4.z, bv4.z, d0, w0) + entry_less(bd4.w, bv4.w, d0, w0);
+            if (m > 32u)
+                r1 += entry_less(bd4.x, bv4.x, d1, w1) + entry_less(bd4.y, bv4.y, d1, w1) +
+                      entry_less(bd4.z, bv4.z, d1, w1) + entry_less(bd4.w, bv4.w, d1, w1);
+        }
+        __syncwarp();
+        if (h0) {
+            bd[r0] = d0;
+            bv[r0] = w0;
+        }
+        if (h1) {
+            bd[r1] = d1;
+            bv[r1] = w1;
+        }
+        __syncwarp();
+    }
+    int p0;
+    if (m == 1u && q.n) {
+        p0 = static_cast<int>(queue_place_few<1>(q, bd, bv, m));
+    } else if (m <= 4u && q.n) {
+        p0 = static_cast<int>(queue_place_few<4>(q, bd, bv, m));
+    } else {
+        p0 = queue_place_many(q, bd, bv, m);
+    }
     const uint32_t total = min(q.n + m, q.cap);
     q.n = total;
     if (static_cast<uint32_t>(p0) < q.hint) q.hint = static_cast<uint32_t>(p0);
     if (q.n >= q.L) {
         q.lb = ent_d(q.e[q.L - 1]);
         uint32_t newn = q.n;
+        #pragma unroll 1
         for (uint32_t base = q.L; base < q.n; base += 32) {
             const uint32_t idx = base + lane;
             const bool dead = idx < q.n && ent_d(q.e[idx]) > q.lb;
