@@ -178,6 +178,21 @@ __global__ void l0_rows_repeat_kernel(const unsigned long long* __restrict__ l0r
     }
 }
 
+// Level-0 rows of at most kPadRow ids at a fixed stride, 0xffffffff past each
+// row's length; one warp per vertex.
+__global__ void l0_pad_kernel(const unsigned long long* __restrict__ l0row, const uint32_t* __restrict__ nbrs,
+                              uint32_t n, uint32_t* __restrict__ pad) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps) {
+        const unsigned long long d = l0row[v];
+        const uint32_t len = static_cast<uint32_t>(d >> kRowLenShift);
+        const uint32_t* row = nbrs + (d & kRowStartMask);
+        uint32_t* out = pad + static_cast<size_t>(v) * kPadRow;
+        for (uint32_t i = lane; i < kPadRow; i += 32) out[i] = i < len ? row[i] : 0xffffffffu;
+    }
+}
+
 // Query order for the persistent schedule: the batch's query indices sorted by
 // queue size, largest first (counting sort over log2 buckets of the queue
 // size; order within a bucket is arbitrary). Work stealing then starts the
@@ -407,6 +422,7 @@ int fill_args(artea_gpu_router* r, SearchArgs* a, const float* d_q, uint32_t nq,
     a->g.vinfo = ix->d_vinfo;
     a->g.nbrs = ix->d_nbrs;
     a->g.l0row = ix->d_l0row;
+    a->g.l0pad = ix->d_l0pad;
     a->g.n = ix->n;
     a->g.dim = ix->dim;
     a->g.top = ix->top;
@@ -435,7 +451,7 @@ int fill_args(artea_gpu_router* r, SearchArgs* a, const float* d_q, uint32_t nq,
     for (int h = 0; h < kMaxGroups; ++h) a->es_thr[h] = r->es_thr[h];
     // The pipelined level-0 loop takes whole rows of distinct ids, <= 64 each
     // (prepare_launch applies the launch's tuning on top).
-    a->l0_pipe = (r->want_pipeline != kNoHash && ix->l0_unique && ix->bl <= 64u) ? 1u : 0u;
+    a->l0_pipe = (r->want_pipeline != kNoHash && ix->d_l0pad) ? 1u : 0u;
     return ARTEA_GPU_OK;
 }
 
@@ -1008,6 +1024,17 @@ int index_finish_l0(artea_gpu_index* ix, const uint32_t* vertex_info, const uint
     dev_free(d_repeat);
     if (e != cudaSuccess) return fail(ARTEA_GPU_ECUDA, "row check failed");
     ix->l0_unique = repeat ? 0u : 1u;
+    if (ix->l0_unique && ix->bl <= kPadRow) {
+        // The fixed-stride copy of the level-0 rows (DeviceGraph::l0pad). It is
+        // only an access path: without the memory for it the CSR rows serve.
+        const size_t ids = static_cast<size_t>(ix->n) * kPadRow;
+        if (dev_alloc(&ix->d_l0pad, ids) == ARTEA_GPU_OK) {
+            l0_pad_kernel<<<std::max(sms, 1) * 8, 256>>>(ix->d_l0row, ix->d_nbrs, ix->n, ix->d_l0pad);
+            if (cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess)
+                return fail(ARTEA_GPU_ECUDA, "level-0 rows failed");
+            ix->bytes += sizeof(uint32_t) * ids;
+        }
+    }
     return ARTEA_GPU_OK;
 }
 
@@ -1091,6 +1118,7 @@ int artea_gpu_index_destroy(artea_gpu_index* ix) {
     dev_free(ix->d_nbrs);
     dev_free(ix->d_offsets);
     dev_free(ix->d_l0row);
+    dev_free(ix->d_l0pad);
     delete ix;
     return ARTEA_GPU_OK;
 }

@@ -31,6 +31,7 @@ struct artea_gpu_index {
     uint32_t* d_nbrs = nullptr;
     uint64_t* d_offsets = nullptr;
     unsigned long long* d_l0row = nullptr;
+    uint32_t* d_l0pad = nullptr;   // level-0 rows at a fixed stride (null: not available)
     const uint64_t* group_ptr[artea_gpu::kMaxGroups] = {};
     uint64_t n_offsets = 0;   // entries of d_offsets (all groups, with their end sentinels)
     uint64_t n_nbrs = 0;      // entries of d_nbrs in use

@@ -34,6 +34,7 @@ constexpr uint32_t kVidMask = 0x7fffffffu;
 constexpr uint32_t kInvalidLevel = 0xffffffffu;
 constexpr uint32_t kEmptySlot = 0xffffffffu;
 constexpr uint32_t kCandBatch = 64;     // candidates evaluated per distance batch
+constexpr uint32_t kPadRow = 64;        // ids per fixed-stride level-0 row (DeviceGraph::l0pad)
 constexpr int kMaxGroups = 64;
 constexpr int kRowLenShift = 40;        // l0row: start in bits 0..39, length in 40..63
 constexpr unsigned long long kRowStartMask = (1ull << kRowLenShift) - 1ull;
@@ -57,7 +58,13 @@ struct DeviceGraph {
     const uint2* __restrict__ vinfo;
     const uint32_t* __restrict__ nbrs;
     const unsigned long long* __restrict__ l0row;
+    // Level-0 rows at a fixed stride: N x kPadRow ids, 0xffffffff past the row's
+    // length, so a row's ids are one dependent load away from its vid instead of
+    // two (descriptor, ids). Null when some row is longer or repeats an id.
+    // (1M x 128, 10,000 queries, queue 400: 13.20 -> 12.56 ms.)
+    const uint32_t* __restrict__ l0pad;
     uint32_t n;
+
     uint32_t dim;
     uint32_t top;      // kInvalidLevel when empty
     uint32_t entry;
@@ -1298,6 +1305,17 @@ __device__ __forceinline__ WarpSmem carve(float* base, uint32_t dim, uint32_t ca
     return s;
 }
 
+// collect_row64_unique for a fixed-stride row (ids0 = slot lane, ids1 = slot 32 +
+// lane), counting the expansion.
+__device__ __forceinline__ uint32_t collect_pad_row(const DeviceGraph& g, Visited& vs, uint32_t ids0, uint32_t ids1,
+                                                    uint32_t* cvid, Counters& ct, int* error) {
+    const uint32_t len = __popc(__ballot_sync(kFull, ids0 != 0xffffffffu)) +
+                         __popc(__ballot_sync(kFull, ids1 != 0xffffffffu));
+    ct.l0_rows++;
+    ct.l0_row_ids += len;
+    return collect_row64_unique(g, vs, ids0, ids1, len, cvid, error);
+}
+
 // ---------------------------------------------------------------------------
 // Level-0 beam search, pipelined across expansions (single_layer_router.hpp:
 // 145-163, beam_loop.hpp:90-119), for graphs whose level-0 rows hold at most 64
@@ -1334,36 +1352,21 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
     if (lane == 0) q.e[0].x |= kExplored;
     __syncwarp();
     q.hint = 1;
-    unsigned long long desc = __ldg(g.l0row + cur);
-    uint32_t len = static_cast<uint32_t>(desc >> kRowLenShift);
-    const uint32_t* row = g.nbrs + (desc & kRowStartMask);
-    uint32_t ids0 = lane < len ? __ldg(row + lane) : 0xffffffffu;
-    uint32_t ids1 = lane + 32 < len ? __ldg(row + lane + 32) : 0xffffffffu;
-    uint32_t cnt = collect_row64_unique(g, vs, ids0, ids1, len, cv, a.error);
-    ct.l0_rows++;
-    ct.l0_row_ids += len;
+    const uint32_t* pad = g.l0pad + lane;
+    uint32_t ids0 = __ldg(pad + static_cast<size_t>(cur) * kPadRow);
+    uint32_t ids1 = __ldg(pad + static_cast<size_t>(cur) * kPadRow + 32);
+    uint32_t cnt = collect_pad_row(g, vs, ids0, ids1, cv, ct, a.error);
     ulonglong2 pre[kBlock];
     dist_preload<kRegs>(g, cv, cnt, pre, l2_next);
     pc.lap(kPhCollect);
     // The predicted entry after the one being expanded: its index (-1: none),
-    // vid, row descriptor and, once loaded, ids.
+    // vid and ids.
     int p2 = -1;
-    uint32_t pf_vid = kVidMask;
-    unsigned long long pf_desc = 0ull;
-    uint32_t pf_ids0 = 0u, pf_ids1 = 0u;
-    bool pf_have_ids = false;
+    uint32_t pf_vid = kVidMask, pf_ids0 = 0u, pf_ids1 = 0u;
     for (uint32_t it = 0;; ++it) {
         if (it > g.n) { set_error(a.error, kErrBound); break; }
         if (cnt) batch_distances<kMetric, kExact, false, kRegs>(g, sm.q, qsq, cv, cd, cnt, st, a.error, &pre);
         ct.dist_evals += cnt;
-        if (p2 >= 0 && !pf_have_ids) {
-            // The predicted entry's descriptor has arrived by now: fetch its ids.
-            const uint32_t len2 = static_cast<uint32_t>(pf_desc >> kRowLenShift);
-            const uint32_t* row2 = g.nbrs + (pf_desc & kRowStartMask);
-            pf_ids0 = lane < len2 ? __ldg(row2 + lane) : 0xffffffffu;
-            pf_ids1 = lane + 32 < len2 ? __ldg(row2 + lane + 32) : 0xffffffffu;
-            pf_have_ids = true;
-        }
         pc.lap(kPhDist);
         const uint32_t m = cnt ? queue_accept(q, cv, cd, cnt, sm.bd, sm.bv) : 0u;
         // The next pop: min(p2, smallest accepted), or termination.
@@ -1392,22 +1395,11 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
         if (go) {
             const bool hit = !take_new && next == pf_vid;
             if (hit) pc.count(kPhPrefetchHits);
-            desc = hit ? pf_desc : __ldg(g.l0row + next);
-            len = static_cast<uint32_t>(desc >> kRowLenShift);
-            row = g.nbrs + (desc & kRowStartMask);
-            if (hit && pf_have_ids) {
-                ids0 = pf_ids0;
-                ids1 = pf_ids1;
-            } else {
-                ids0 = lane < len ? __ldg(row + lane) : 0xffffffffu;
-                ids1 = lane + 32 < len ? __ldg(row + lane + 32) : 0xffffffffu;
-            }
-            pf_have_ids = false;
+            ids0 = hit ? pf_ids0 : __ldg(pad + static_cast<size_t>(next) * kPadRow);
+            ids1 = hit ? pf_ids1 : __ldg(pad + static_cast<size_t>(next) * kPadRow + 32);
             pc.lap(kPhPop);
             // The current candidates are in bd/bv now: cv takes the next row's.
-            ncnt = collect_row64_unique(g, vs, ids0, ids1, len, cv, a.error);
-            ct.l0_rows++;
-            ct.l0_row_ids += len;
+            ncnt = collect_pad_row(g, vs, ids0, ids1, cv, ct, a.error);
             dist_preload<kRegs>(g, cv, ncnt, pre, l2_next);
             pc.lap(kPhCollect);
         }
@@ -1422,7 +1414,8 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
         if (p2 >= 0) {
             q.hint = static_cast<uint32_t>(p2);
             pf_vid = q.e[p2].x & kVidMask;
-            pf_desc = __ldg(g.l0row + pf_vid);
+            pf_ids0 = __ldg(pad + static_cast<size_t>(pf_vid) * kPadRow);
+            pf_ids1 = __ldg(pad + static_cast<size_t>(pf_vid) * kPadRow + 32);
         } else {
             q.hint = q.n;
             pf_vid = kVidMask;
