@@ -49,14 +49,14 @@ struct Tuning {
     uint32_t stage = 0;  // 0: rows read with vector loads; kStageRows: TMA-staged in shared memory
     uint32_t pf = 0;     // pipelined level-0 loop: 1 = the second pass's rows are prefetched into L2
     uint32_t pipe = 1;   // pipelined level-0 loop where the graph allows it (0: one expansion at a time)
-    uint32_t wpq = 1;    // warps per query: > 1 = cooperative kernel, a CTA of wpq warps per query
+    uint32_t team = 0;   // row warps of the team kernel (2, 4 or 8; a CTA searches a query); 0: a warp per query
     uint32_t slack = 0;  // queue layout: 0 = 2L entries per search; > 0 = compact, max queue + slack
                          // entries, a query that could lose a live entry is rerun at 2L
 };
 
 // One field per tuning component (graph keys, the launch-shape cache).
 uint64_t tuning_bits(const Tuning& t) {
-    return (static_cast<uint64_t>(t.slack) << 44) | (static_cast<uint64_t>(t.wpq) << 40) |
+    return (static_cast<uint64_t>(t.slack) << 44) | (static_cast<uint64_t>(t.team) << 40) |
            (static_cast<uint64_t>(t.warps) << 32) |
            (static_cast<uint64_t>(t.pipe) << 29) |
            (static_cast<uint64_t>(t.pf) << 28) |
@@ -239,9 +239,8 @@ using KernelFn = void (*)(SearchArgs);
 // 2 = 96 (CTAs of at most 4 warps) (persistent only); stage: rows staged in
 // shared memory by TMA.
 // Kernels with the pipelined level-0 loop exist for the 96- and 128-register
-// budgets (the 128-register kernel always carries it; it falls back to one
-// expansion at a time on graphs that do not allow it); the others run one
-// expansion at a time.
+// budgets; the others run one expansion at a time, as the 96-register one does
+// for a 128-register launch on a graph without fixed-stride rows.
 template <int kMetric, bool kExact, bool kStage>
 KernelFn pick_persistent_s(uint32_t regs, bool pipe) {
     switch (regs) {
@@ -249,7 +248,10 @@ KernelFn pick_persistent_s(uint32_t regs, bool pipe) {
         case 2:
             if (pipe) return kStage ? nullptr : search_persistent_kernel<kMetric, kExact, 96, false, true>;
             return search_persistent_kernel<kMetric, kExact, 96, kStage>;
-        case 3: return kStage ? nullptr : search_persistent_kernel<kMetric, kExact, 128, false, true>;
+        case 3:
+            if (kStage) return nullptr;
+            return pipe ? search_persistent_kernel<kMetric, kExact, 128, false, true>
+                        : search_persistent_kernel<kMetric, kExact, 96, false>;
         default: return search_persistent_kernel<kMetric, kExact, 85, kStage>;
     }
 }
@@ -276,19 +278,35 @@ KernelFn pick_kernel_m(bool exact, bool persistent, uint32_t regs, bool stage, b
     return exact ? search_plain_kernel<kMetric, true, false> : search_plain_kernel<kMetric, false, false>;
 }
 
-template <int kMetric>
-KernelFn pick_coop_m(bool exact, uint32_t wpq) {
-    if (wpq == 2) return exact ? search_coop_kernel<kMetric, true, 2> : search_coop_kernel<kMetric, false, 2>;
-    if (wpq == 4) return exact ? search_coop_kernel<kMetric, true, 4> : search_coop_kernel<kMetric, false, 4>;
-    return nullptr;
+// Router option warps_per_query: 1 = a warp per query, 2 = a small team (2 or 4
+// row warps), 4 = a large one (8).
+uint32_t wpq_of(uint32_t team) { return team == 0 ? 1u : (team == 8 ? 4u : 2u); }
+
+// pad: level 0 split over the team (graphs with fixed-stride rows); without it
+// the teams of 4 and 8 only split the distance batches.
+template <int kMetric, bool kExact>
+KernelFn pick_team_e(uint32_t team, bool pad) {
+    switch (team) {
+        case 2: return pad ? search_team_kernel<kMetric, kExact, 2, true> : nullptr;
+        case 4: return pad ? search_team_kernel<kMetric, kExact, 4, true> : search_team_kernel<kMetric, kExact, 4, false>;
+        case 8: return pad ? search_team_kernel<kMetric, kExact, 8, true> : search_team_kernel<kMetric, kExact, 8, false>;
+        default: return nullptr;
+    }
 }
 
-KernelFn pick_coop(int metric, bool exact, uint32_t wpq) {
-    switch (metric) {
-        case ARTEA_GPU_EUCLIDEAN_SQR: return pick_coop_m<ARTEA_GPU_EUCLIDEAN_SQR>(exact, wpq);
-        case ARTEA_GPU_EUCLIDEAN: return pick_coop_m<ARTEA_GPU_EUCLIDEAN>(exact, wpq);
-        case ARTEA_GPU_COSINE: return pick_coop_m<ARTEA_GPU_COSINE>(exact, wpq);
-        case ARTEA_GPU_DOT: return pick_coop_m<ARTEA_GPU_DOT>(exact, wpq);
+template <int kMetric>
+KernelFn pick_team_m(bool exact, uint32_t team, bool pad) {
+    return exact ? pick_team_e<kMetric, true>(team, pad) : pick_team_e<kMetric, false>(team, pad);
+}
+
+KernelFn pick_team(const artea_gpu_router* r, uint32_t team) {
+    const bool exact = r->mode == ARTEA_GPU_MODE_EXACT;
+    const bool pad = r->idx->d_l0pad && r->want_pipeline != kNoHash;
+    switch (r->metric) {
+        case ARTEA_GPU_EUCLIDEAN_SQR: return pick_team_m<ARTEA_GPU_EUCLIDEAN_SQR>(exact, team, pad);
+        case ARTEA_GPU_EUCLIDEAN: return pick_team_m<ARTEA_GPU_EUCLIDEAN>(exact, team, pad);
+        case ARTEA_GPU_COSINE: return pick_team_m<ARTEA_GPU_COSINE>(exact, team, pad);
+        case ARTEA_GPU_DOT: return pick_team_m<ARTEA_GPU_DOT>(exact, team, pad);
         default: return nullptr;
     }
 }
@@ -386,16 +404,16 @@ int persistent_shape(artea_gpu_router* r, const Tuning& t, LaunchShape* s) {
     }
     if ((t.regs == 2 || t.regs == 3) && t.warps > 4)
         return fail(ARTEA_GPU_EINVAL, "register budgets 96 and 128 allow at most 4 warps per CTA");
-    const bool coop = t.wpq > 1;
-    KernelFn fn = coop ? pick_coop(r->metric, r->mode == ARTEA_GPU_MODE_EXACT, t.wpq)
+    const bool team = t.team != 0;
+    KernelFn fn = team ? pick_team(r, t.team)
                        : pick_kernel(r->metric, r->mode == ARTEA_GPU_MODE_EXACT, true, t.regs, t.stage != 0,
                                      t.pipe != 0);
     if (!fn)
         return fail(ARTEA_GPU_EINVAL, "no kernel for this combination (staged rows with the 128-register budget, or "
                                       "the pipelined loop with a budget below 96)");
-    const uint32_t cta_threads = coop ? t.wpq * 32 : t.warps * 32;
+    const uint32_t cta_threads = team ? (t.team + 1) * 32 : t.warps * 32;
     const uint32_t cap = launch_cap(r, t);
-    const uint32_t smem = coop ? smem_bytes_per_warp(r->idx->dim, cap, t.vh_bits) + kCoopWords * 4
+    const uint32_t smem = team ? smem_bytes_per_warp(r->idx->dim, cap, t.vh_bits) + kCoopWords * 4
                                : smem_bytes_per_warp(r->idx->dim, cap, t.vh_bits, t.stage) * t.warps;
     if (smem > 227u * 1024u) return fail(ARTEA_GPU_EINVAL, "persistent CTA needs more than 227 KB shared memory");
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -405,9 +423,9 @@ int persistent_shape(artea_gpu_router* r, const Tuning& t, LaunchShape* s) {
                                                            static_cast<int>(cta_threads), smem));
     if (per_sm <= 0) return fail(ARTEA_GPU_EINVAL, "persistent kernel does not fit on an SM (queue too large?)");
     if (r->want_ctas_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(r->want_ctas_per_sm));
-    s->warps_per_cta = coop ? t.wpq : t.warps;
+    s->warps_per_cta = team ? t.team + 1 : t.warps;
     s->ctas = static_cast<uint32_t>(per_sm) * static_cast<uint32_t>(r->num_sms);
-    s->slots = coop ? s->ctas : s->ctas * t.warps;   // one visited slot per search in flight
+    s->slots = team ? s->ctas : s->ctas * t.warps;   // one visited slot per search in flight
     r->shapes[key] = *s;
     return ARTEA_GPU_OK;
 }
@@ -474,20 +492,17 @@ struct Prepared {
 
 int prepare_launch(artea_gpu_router* r, SearchArgs a, bool persistent, const Tuning& t, Prepared* p) {
     const bool exact = r->mode == ARTEA_GPU_MODE_EXACT;
-    const bool coop = persistent && t.wpq > 1;
+    const bool team = persistent && t.team != 0;
     // The pipelined loop runs where the graph allows it, the router and the
     // tuning ask for it, and the kernel carries it (persistent: the 96- and
-    // 128-register kernels with vector loads; the 128-register kernel always
-    // carries it and falls back on its own).
+    // 128-register kernels with vector loads).
     const bool staged = persistent && t.stage != 0;
-    const bool has_pipe = !coop && !staged && (persistent ? t.regs == 2 || t.regs == 3 : true);
+    const bool has_pipe = !team && !staged && (persistent ? t.regs == 2 || t.regs == 3 : true);
     a.l0_pipe = (a.l0_pipe && t.pipe && has_pipe) ? 1u : 0u;
-    const bool pipe_kernel = a.l0_pipe || (persistent && !coop && t.regs == 3);
-    KernelFn fn = coop ? pick_coop(r->metric, exact, t.wpq)
-                       : pick_kernel(r->metric, exact, persistent, t.regs, staged, pipe_kernel);
+    KernelFn fn = team ? pick_team(r, t.team)
+                       : pick_kernel(r->metric, exact, persistent, t.regs, staged, a.l0_pipe != 0);
     if (!fn) return fail(ARTEA_GPU_EINVAL, "no kernel for this metric and option combination");
-    // The compact queue layout: one-warp persistent kernels only.
-    const bool compact = persistent && !coop && t.slack != 0;
+    const bool compact = persistent && t.slack != 0;
     a.cap = compact ? launch_cap(r, t) : r->cap;
     a.compact = compact ? 1u : 0u;
     if (compact) {
@@ -502,11 +517,11 @@ int prepare_launch(artea_gpu_router* r, SearchArgs a, bool persistent, const Tun
     if (!a.vk_bits) return fail(ARTEA_GPU_EINVAL, "visited table too small for N");
     p->fn = fn;
     p->persistent = persistent;
-    if (coop) {
+    if (team) {
         LaunchShape s;
         if (int rc = persistent_shape(r, t, &s)) return rc;
         p->grid = std::min(s.ctas, a.nq);
-        p->threads = t.wpq * 32;
+        p->threads = (t.team + 1) * 32;
         p->smem = smem_bytes_per_warp(r->idx->dim, a.cap, t.vh_bits) + kCoopWords * 4;
         if (int rc = ensure_slots(r, p->grid)) return rc;
     } else if (persistent) {
@@ -685,8 +700,8 @@ bool tuning_file_load(const std::string& path, const std::string& fkey, Tuning* 
         unsigned w, b, rg, st, pf, pp, q, sl;
         if (std::sscanf(line, "%599s %u %u %u %u %u %u %u %u", k, &w, &b, &rg, &st, &pf, &pp, &q, &sl) == 9 &&
             fkey == k && rg <= 3 && (st == 0 || st == kStageRows) && pf <= 1 && pp <= 1 && w >= 1 && w <= 8 &&
-            b <= 12 && (q == 1 || q == 2 || q == 4) && sl <= 4096) {
-            t->wpq = q;
+            b <= 12 && (q == 0 || q == 2 || q == 4 || q == 8) && sl <= 4096) {
+            t->team = q;
             t->slack = sl;
             t->warps = w;
             t->vh_bits = b;
@@ -713,7 +728,7 @@ void tuning_file_store(const std::string& path, const std::string& fkey, const T
     FILE* f = std::fopen(path.c_str(), "a");
     if (!f) return;
     std::fprintf(f, "%s %u %u %u %u %u %u %u %u\n", fkey.c_str(), t.warps, t.vh_bits, t.regs, t.stage, t.pf, t.pipe,
-                 t.wpq, t.slack);
+                 t.team, t.slack);
     std::fclose(f);
 }
 
@@ -731,7 +746,7 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
     const bool fixed_pf = r->want_prefetch != 0 || !a.l0_pipe;
     const uint32_t pf_fixed = r->want_prefetch == 16 ? 1u : 0u;
     if (r->want_wpq > 1 && r->want_vh_bits) {
-        t.wpq = r->want_wpq;
+        t.team = r->want_wpq == 4 ? 8u : 4u;
         t.warps = 1;
         t.vh_bits = hash_bits_of(r->want_vh_bits);
         t.regs = 2;
@@ -789,8 +804,8 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
     best.pf = pf_choices[0];
     best.pipe = pipe_choices.back();
     auto time_candidate = [&](const Tuning& c) {
-        if (r->want_wpq && c.wpq != r->want_wpq) return;
-        if (c.slack && (c.wpq > 1 || c.stage)) return;   // compact queues: one-warp kernels, vector loads
+        if (r->want_wpq && wpq_of(c.team) != r->want_wpq) return;
+        if (c.slack && c.stage) return;        // compact queues: vector loads
         if (c.stage && c.pf) return;           // staged rows use the one-expansion loop
         if (c.stage && c.regs == 3) return;    // no staged 128-register kernel
         if ((c.regs == 2 || c.regs == 3) && c.warps > 4) return;
@@ -843,26 +858,27 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
                         c.slack = slack;
                         time_candidate(c);
                     }
-    // 1b. warps per query: the cooperative kernel (96 registers, vector
-    // loads, one expansion at a time) at every table size.
-    std::vector<uint32_t> wpq_choices = {2, 4};
-    if (r->want_wpq) wpq_choices = r->want_wpq > 1 ? std::vector<uint32_t>{r->want_wpq} : std::vector<uint32_t>{};
-    if (r->want_warps || r->want_regs || r->want_stage || r->want_prefetch || r->want_pipeline == 1)
-        wpq_choices.clear();   // those options describe the one-warp kernels
-    for (uint32_t q : wpq_choices)
-        for (uint32_t b : bit_choices) {
-            Tuning c;
-            c.wpq = q;
-            c.warps = 1;
-            c.vh_bits = b;
-            c.regs = 2;
-            c.stage = 0;
-            c.pf = 0;
-            c.pipe = 0;
-            time_candidate(c);
-        }
+    // 1b. warps per query: the team kernel at every team and table size.
+    std::vector<uint32_t> team_choices = {2, 4, 8};
+    if (r->want_wpq == 1 || r->want_warps || r->want_regs || r->want_stage || r->want_prefetch ||
+        r->want_pipeline == 1)
+        team_choices.clear();   // those options describe the one-warp kernels
+    for (uint32_t slack : slack_choices)
+        for (uint32_t g : team_choices)
+            for (uint32_t b : bit_choices) {
+                Tuning c;
+                c.team = g;
+                c.warps = 1;
+                c.vh_bits = b;
+                c.regs = 2;
+                c.stage = 0;
+                c.pf = 0;
+                c.pipe = 0;
+                c.slack = slack;
+                time_candidate(c);
+            }
     // 2. rows loaded ahead, at the best shape (pipelined loop only).
-    for (size_t i = 1; i < pf_choices.size() && best.pipe && best.wpq == 1 && a.l0_pipe; ++i) {
+    for (size_t i = 1; i < pf_choices.size() && best.pipe && !best.team && a.l0_pipe; ++i) {
         Tuning c = best;
         c.pf = pf_choices[i];
         time_candidate(c);
@@ -1351,7 +1367,7 @@ int artea_gpu_router_tuning_ext(const artea_gpu_router* r, uint32_t* pipeline, u
     *pipeline = r->last_pipe ? 1u : 0u;
     *prefetch_rows = r->last.pf ? 16u : 8u;
     *ordered = r->last_ordered ? 1u : 0u;
-    *warps_per_query = r->last.wpq;
+    *warps_per_query = wpq_of(r->last.team);
     return ARTEA_GPU_OK;
 }
 

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kProbeBudgetThreads, 5) probe_trace_kernel(Sea
         if (lane_id() == 0) qi = atomicAdd(a.next_query, 1u);
         qi = __shfl_sync(kFull, qi, 0);
         if (qi >= a.nq) break;
-        search_one<kMetric, kExact, false, false, 1, false, true>(a, qi, slot, sm);
+        search_one<kMetric, kExact, false, false, 0, false, true>(a, qi, slot, sm);
     }
 }
 

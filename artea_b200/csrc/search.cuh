@@ -64,7 +64,6 @@ struct DeviceGraph {
     // (1M x 128, 10,000 queries, queue 400: 13.20 -> 12.56 ms.)
     const uint32_t* __restrict__ l0pad;
     uint32_t n;
-
     uint32_t dim;
     uint32_t top;      // kInvalidLevel when empty
     uint32_t entry;
@@ -115,7 +114,7 @@ struct SearchArgs {
     uint32_t compact;         // queue capacity may be below 2L: a query that could lose a live
                               // entry is abandoned and listed in overflow for the full-capacity rerun
     uint32_t* __restrict__ overflow;   // [count, rerun counter, query indices...] (compact only)
-    uint32_t l0_pipe;         // level-0 rows hold <= 64 distinct ids: pipelined level-0 loop
+    uint32_t l0_pipe;         // the launch takes a kernel with the pipelined level-0 loop (needs g.l0pad)
     uint32_t pf_l2;           // pipelined loop: also prefetch the second pass's rows into L2
     const uint32_t* __restrict__ order;   // persistent schedule: query order (null: 0..nq-1)
     TraceArgs tr;             // kernels compiled with kTrace only
@@ -186,6 +185,7 @@ template <bool kExact>
 __device__ float query_sqnorm(const float* __restrict__ q, uint32_t dim) {
     const int g = lane_id() & 3;
     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+    #pragma unroll 1
     for (uint32_t c = 0; c < dim; c += 16) {
         const float4 v = *reinterpret_cast<const float4*>(q + c + 4 * g);
         a0 = fmaf(v.x, v.x, a0); a1 = fmaf(v.y, v.y, a1);
@@ -256,6 +256,7 @@ __device__ __forceinline__ void bulk_row_copy(uint32_t dst, const float* src, ui
 
 // Bounded wait for the phase with the given parity; false if it never came.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
+    #pragma unroll 1
     for (uint32_t i = 0; i < kWaitBound; ++i) {
         uint32_t ok;
         asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -330,6 +331,7 @@ __device__ void batch_distances(const DeviceGraph& g, const float* __restrict__ 
     const uint32_t dim = g.dim;
     const uint32_t nchunks = dim >> 4;
     const uint32_t sstride = dim + kStagePad;
+    #pragma unroll 1
     for (uint32_t p = 8u * pass0; p < cnt; p += 8u * stride) {
         const uint32_t idx = p + r;
         const bool valid = idx < cnt;
@@ -360,6 +362,7 @@ __device__ void batch_distances(const DeviceGraph& g, const float* __restrict__ 
         }
         const float* qq = q + 4 * gi;
         f32x2 A01 = 0ull, A23 = 0ull;   // L2: diff^2; dot/cos: q*x   (+0.0f pairs)
+        #pragma unroll 1
         for (uint32_t cb = 0; cb < nchunks; cb += kBlock) {
             ulonglong2 x[kBlock];
             if (kPre && p == 0 && cb == 0) {
@@ -397,34 +400,194 @@ __device__ void batch_distances(const DeviceGraph& g, const float* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// Cooperative distances (warps per query > 1). A CTA of kW warps searches one
-// query: warp 0 runs the search; at every distance batch it publishes the
-// candidates here and all kW warps take the 8-row passes in turn (warp w:
-// passes w, w + kW, ...), each row by one warp with the same code, so the
-// distances are bit-identical to one warp's. Two named-barrier phases per
-// batch: start (the batch is published) and done (every distance is
-// written). After its last query warp 0 publishes quit at a start barrier.
+// Distances of a row warp's few rows (team search). One warp per scheduler
+// issues an instruction every 4-6 cycles here, so what counts is instructions:
+// lanes without a row of their own repeat the last one (the same addresses, no
+// extra traffic) instead of being masked, and rows are loaded apart from the
+// arithmetic, ahead of it.
 // ---------------------------------------------------------------------------
+template <int kMetric, bool kExact>
+__device__ __forceinline__ float finish_distance(float res, float qsq, float xsq) {
+    if (kMetric == ARTEA_GPU_EUCLIDEAN) return __fsqrt_rn(res);
+    if (kMetric == ARTEA_GPU_DOT) return -res;
+    if (kMetric == ARTEA_GPU_COSINE) {
+        // utils/simd_distance.hpp:263-274
+        const float denom = __fsqrt_rn(__fmul_rn(qsq, xsq));
+        return denom > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(res, denom)) : 1.0f;
+    }
+    return res;
+}
+
+// A row warp's registers for rows loaded ahead of their arithmetic.
+typedef f32x2 RowRegs[16];
+
+// Rows cvid[p, min(p + 8, cnt)) of at most kBlock chunks (kN: their number, or 0
+// for nchunks), 4 lanes a row as in batch_distances; cnt > p.
+template <int kN>
+__device__ __forceinline__ void row8_load(const DeviceGraph& g, const uint32_t* cvid, uint32_t p, uint32_t cnt,
+                                          uint32_t nchunks, RowRegs& x) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t vid = cvid[min(p + (lane >> 2), cnt - 1u)];
+    const float* row = g.vecs + static_cast<size_t>(vid) * g.dim + 4u * (lane & 3u);
+#pragma unroll
+    for (int k = 0; k < (kN ? kN : kBlock); ++k) {
+        if (kN || static_cast<uint32_t>(k) < nchunks) {
+            const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(row + 16 * k));
+            x[2 * k] = w.x;
+            x[2 * k + 1] = w.y;
+        }
+    }
+}
+
+template <int kMetric, bool kExact, int kN>
+__device__ __forceinline__ void row8_distance(const DeviceGraph& g, const float* __restrict__ q, float qsq,
+                                              const uint32_t* cvid, float* cdist, uint32_t p, uint32_t cnt,
+                                              uint32_t nchunks, const RowRegs& x) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t idx = p + (lane >> 2);
+    const float xsq = kMetric == ARTEA_GPU_COSINE ? __ldg(g.xsq + cvid[min(idx, cnt - 1u)]) : 1.0f;
+    const float* qq = q + 4u * (lane & 3u);
+    f32x2 A01 = 0ull, A23 = 0ull;
+#pragma unroll
+    for (int k = 0; k < (kN ? kN : kBlock); ++k)
+        if (kN || static_cast<uint32_t>(k) < nchunks)
+            accumulate<kMetric>(make_ulonglong2(x[2 * k], x[2 * k + 1]),
+                                *reinterpret_cast<const ulonglong2*>(qq + 16 * k), A01, A23);
+    const float res = finish_distance<kMetric, kExact>(fold16<kExact>(lo32(A01), hi32(A01), lo32(A23), hi32(A23)), qsq,
+                                                       xsq);
+    if (idx < cnt && (lane & 3u) == 0u) cdist[idx] = res;
+}
+
+// Rows of more than kBlock chunks: 16 lanes a row, lane j owning the reference's
+// AVX-512 lane j (element 16c + j of every chunk c), so a lane keeps 32 chunks in
+// flight, one register each (chunk k of a block in half k & 1 of x[k / 2]); two
+// rows a pass. The fold's xor steps (8, 4, 2, 1) are fold16's tree (FAST: 1, 2,
+// 4, 8, fold16<false>'s order), so distances are bit-identical.
+constexpr uint32_t kWideBlock = 32;
+
+// Block cb (in chunks) of rows cvid[p, min(p + 2, cnt)); cnt > p.
+__device__ __forceinline__ void wide_load(const DeviceGraph& g, const uint32_t* cvid, uint32_t p, uint32_t cnt,
+                                          uint32_t cb, RowRegs& x) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t left = (g.dim >> 4) - cb;
+    const uint32_t vid = cvid[min(p + (lane >> 4), cnt - 1u)];
+    const float* row = g.vecs + static_cast<size_t>(vid) * g.dim + (lane & 15u) + 16u * cb;
+#pragma unroll
+    for (int k = 0; k < static_cast<int>(kWideBlock); k += 2) {
+        float f0 = 0.0f, f1 = 0.0f;
+        if (static_cast<uint32_t>(k) < left) f0 = __ldg(row + 16 * k);
+        if (static_cast<uint32_t>(k) + 1u < left) f1 = __ldg(row + 16 * k + 16);
+        x[k / 2] = static_cast<f32x2>(__float_as_uint(f0)) | (static_cast<f32x2>(__float_as_uint(f1)) << 32);
+    }
+}
+
+template <int kMetric, bool kExact>
+__device__ __forceinline__ void wide_distance(const DeviceGraph& g, const float* __restrict__ q, float qsq,
+                                              const uint32_t* cvid, float* cdist, uint32_t p, uint32_t cnt,
+                                              RowRegs& x) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t j = lane & 15u;
+    const uint32_t nchunks = g.dim >> 4;
+    const uint32_t idx = p + (lane >> 4);
+    const float xsq = kMetric == ARTEA_GPU_COSINE ? __ldg(g.xsq + cvid[min(idx, cnt - 1u)]) : 1.0f;
+    float acc = 0.0f;
+    #pragma unroll 1
+    for (uint32_t cb = 0; cb < nchunks; cb += kWideBlock) {
+        if (cb) wide_load(g, cvid, p, cnt, cb, x);
+#pragma unroll
+        for (int k = 0; k < static_cast<int>(kWideBlock); ++k) {
+            if (cb + k < nchunks) {
+                const float y = q[16u * (cb + k) + j], v = (k & 1) ? hi32(x[k / 2]) : lo32(x[k / 2]);
+                if (kMetric == ARTEA_GPU_EUCLIDEAN_SQR || kMetric == ARTEA_GPU_EUCLIDEAN) {
+                    const float d = __fsub_rn(y, v);
+                    acc = __fmaf_rn(d, d, acc);
+                } else {
+                    acc = __fmaf_rn(y, v, acc);
+                }
+            }
+        }
+    }
+    if (kExact) {
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(kFull, acc, off));
+    } else {
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) acc = __fadd_rn(acc, __shfl_xor_sync(kFull, acc, off));
+    }
+    const float res = finish_distance<kMetric, kExact>(acc, qsq, xsq);
+    if (idx < cnt && j == 0u) cdist[idx] = res;
+}
+
+// A row warp's rows of one pass, by width (128 and 96, the benchmark's, have
+// their own code).
+__device__ __forceinline__ void slice_load(const DeviceGraph& g, const uint32_t* cvid, uint32_t p, uint32_t cnt,
+                                           RowRegs& x) {
+    const uint32_t nchunks = g.dim >> 4;
+    if (nchunks == 8u) row8_load<8>(g, cvid, p, cnt, nchunks, x);
+    else if (nchunks == 6u) row8_load<6>(g, cvid, p, cnt, nchunks, x);
+    else if (nchunks <= kBlock) row8_load<0>(g, cvid, p, cnt, nchunks, x);
+    else wide_load(g, cvid, p, cnt, 0, x);
+}
+
+template <int kMetric, bool kExact>
+__device__ __forceinline__ void slice_distance(const DeviceGraph& g, const float* __restrict__ q, float qsq,
+                                               const uint32_t* cvid, float* cdist, uint32_t p, uint32_t cnt,
+                                               RowRegs& x) {
+    const uint32_t nchunks = g.dim >> 4;
+    if (nchunks == 8u) row8_distance<kMetric, kExact, 8>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
+    else if (nchunks == 6u) row8_distance<kMetric, kExact, 6>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
+    else if (nchunks <= kBlock) row8_distance<kMetric, kExact, 0>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
+    else wide_distance<kMetric, kExact>(g, q, qsq, cvid, cdist, p, cnt, x);
+}
+
+// ---------------------------------------------------------------------------
+// Team search (warps per query > 1): a CTA of kG row warps and one queue warp
+// (warp 0, the leader) searches one query. The leader publishes commands here
+// and all warps meet at a named barrier. kCmdDist: every warp of the CTA takes
+// the 8-row passes of a distance batch in turn (warp w: passes w, w + W, ...;
+// upper levels, and level 0 of graphs without fixed-stride rows), each row by
+// one warp with the same code, so distances are bit-identical to one warp's.
+// kCmdLevel0: the row warps enter the level-0 loop (l0_team_rows) and leave it
+// when the leader ends it. kCmdQuit: no queries are left.
+// ---------------------------------------------------------------------------
+enum : uint32_t { kCmdDist = 0, kCmdLevel0 = 1, kCmdQuit = 2 };
+
 struct CoopCtl {
     const uint32_t* cvid;
     float* cdist;
     uint32_t cnt;
     float qsq;
-    uint32_t quit;
-    uint32_t pad[3];
+    uint32_t cmd;
+    uint32_t next;      // level 0: vertex to expand (kVidMask: the loop ends)
+    uint32_t pf;        // level 0: vertex expected to be expanded after it (kVidMask: none)
+    uint32_t list_n;    // level 0: ids put in the visited bitset since the last clear
+    uint32_t evals;     // level 0: distance evaluations
+    uint32_t row_ids;   // level 0: ids in the rows expanded
+    uint32_t pad[4];
+    uint32_t spec[kPadRow];   // level 0: unvisited ids of the expected row, one slice per row warp
 };
 constexpr uint32_t kCoopWords = sizeof(CoopCtl) / 4;
-constexpr int kCoopBarrier = 1;
+static_assert(sizeof(CoopCtl) % 16 == 0, "the control block keeps the regions after it aligned");
+constexpr int kCoopBarrier = 1;   // commands: every warp of the team waits
+constexpr int kRowsBarrier = 2;   // level 0, A: the row warps have written (they do not wait)
+constexpr int kNextBarrier = 3;   // level 0, B: the leader has published (it does not wait)
 
 __device__ __forceinline__ void coop_barrier(int warps) {
     asm volatile("barrier.sync %0, %1;" ::"r"(kCoopBarrier), "r"(warps * 32) : "memory");
 }
+__device__ __forceinline__ void team_arrive(int barrier, int warps) {
+    asm volatile("barrier.arrive %0, %1;" ::"r"(barrier), "r"(warps * 32) : "memory");
+}
+__device__ __forceinline__ void team_wait(int barrier, int warps) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(barrier), "r"(warps * 32) : "memory");
+}
 
-template <int kMetric, bool kExact, bool kStage, int kW>
+// kG: row warps of the team (0: one warp searches alone).
+template <int kMetric, bool kExact, bool kStage, int kG>
 __device__ __forceinline__ void dist_call(const DeviceGraph& g, const float* __restrict__ q, float qsq,
                                           const uint32_t* cvid, float* cdist, uint32_t cnt, Stage& st, int* error,
                                           CoopCtl* coop) {
-    if (kW == 1) {
+    if (kG == 0) {
         batch_distances<kMetric, kExact, kStage>(g, q, qsq, cvid, cdist, cnt, st, error);
         return;
     }
@@ -433,33 +596,11 @@ __device__ __forceinline__ void dist_call(const DeviceGraph& g, const float* __r
         coop->cdist = cdist;
         coop->cnt = cnt;
         coop->qsq = qsq;
-        coop->quit = 0u;
+        coop->cmd = kCmdDist;
     }
-    coop_barrier(kW);   // start
-    batch_distances<kMetric, kExact, false, false, true>(g, q, qsq, cvid, cdist, cnt, st, error, nullptr, 0u, kW);
-    coop_barrier(kW);   // done
-}
-
-// The other warps of a cooperative CTA: take passes of each published batch
-// until warp 0 publishes quit.
-template <int kMetric, bool kExact, int kW>
-__device__ void coop_helper(const DeviceGraph& g, const float* __restrict__ q, CoopCtl* coop, int warp, int* error) {
-    Stage st;
-    st.buf = nullptr;
-    st.mbar = 0u;
-    st.phase = 0u;
-    for (;;) {
-        coop_barrier(kW);   // start
-        const uint32_t quit = coop->quit;
-        const uint32_t cnt = coop->cnt;
-        const uint32_t* cvid = coop->cvid;
-        float* cdist = coop->cdist;
-        const float qsq = coop->qsq;
-        if (quit) break;
-        batch_distances<kMetric, kExact, false, false, true>(g, q, qsq, cvid, cdist, cnt, st, error, nullptr,
-                                                            static_cast<uint32_t>(warp), kW);
-        coop_barrier(kW);   // done
-    }
+    coop_barrier(kG + 1);   // start
+    batch_distances<kMetric, kExact, false, false, true>(g, q, qsq, cvid, cdist, cnt, st, error, nullptr, 0u, kG + 1);
+    coop_barrier(kG + 1);   // done
 }
 
 // ---------------------------------------------------------------------------
@@ -491,6 +632,7 @@ constexpr uint32_t kAltFlag = 0x8000u;          // slot holds an id whose first 
 // 15 bits (table too small for n).
 __host__ __device__ inline uint32_t visited_kbits(uint32_t n, uint32_t table_log) {
     uint32_t kb = 1;
+    #pragma unroll 1
     while (kb < 32 && (1ull << kb) < n) ++kb;
     if (table_log == 0) return kb;
     const uint32_t tbits = table_log + 1;
@@ -582,6 +724,7 @@ __device__ __forceinline__ int table_try(const Visited& vs, const TableWalk& w) 
 // by another lane, so the loop ends within the 8 slots of the two buckets.
 __device__ __forceinline__ int table_test_insert(const Visited& vs, uint32_t vid) {
     const TableWalk w = table_walk(vs, vid);
+    #pragma unroll 1
     for (int step = 0; step < 24; ++step) {
         const int r = table_try(vs, w);
         if (r >= 0) return r;
@@ -630,6 +773,7 @@ __device__ __forceinline__ void table_test_insert2(const Visited& vs, uint32_t v
                                                    int* r0, int* r1) {
     const TableWalk w0 = table_walk(vs, a0 ? v0 : 0u), w1 = table_walk(vs, a1 ? v1 : 0u);
     int t0 = a0 ? -1 : -2, t1 = a1 ? -1 : -2;
+    #pragma unroll 1
     for (int step = 0; step < 24 && (t0 == -1 || t1 == -1); ++step) {
         if (t0 == -1) t0 = table_try(vs, w0);
         if (t1 == -1) t1 = table_try(vs, w1);
@@ -673,11 +817,46 @@ __device__ __forceinline__ void visited_test_and_set2(Visited& vs, uint32_t v0, 
     *new1 = n1;
 }
 
+// Whether an id is unvisited, without marking it. While other warps insert, an
+// id they are inserting may still read as unvisited.
+__device__ __forceinline__ bool visited_open(const Visited& vs, uint32_t vid) {
+    if (vs.tbits) {
+        const TableWalk w = table_walk(vs, vid);
+        const uint2 ba = vs.tab[w.a];
+        const uint2 bb = w.b != 0xffffffffu ? vs.tab[w.b] : make_uint2(0u, 0u);
+        if (bucket_match(ba, w.q * 0x10001u) | bucket_match(bb, (w.q | kAltFlag) * 0x10001u)) return false;
+        if (ba.y >= kHighFree || bb.y >= kHighFree) return true;
+    }
+    return !((__ldcg(vs.bits + (vid >> 5)) >> (vid & 31)) & 1u);
+}
+
+// test_and_set for one id per lane of one warp of a team, other warps doing
+// the same for other ids: the ids put in the bitset are listed through the
+// team's shared count (which may pass list_cap: the list then overflowed).
+__device__ __forceinline__ bool team_test_and_set(const Visited& vs, uint32_t* list_n, uint32_t vid, bool act) {
+    bool is_new = false;
+    if (act) {
+        const int t = vs.tbits ? table_test_insert(vs, vid) : 2;
+        is_new = t == 0;
+        if (t == 2) {
+            const uint32_t mask = 1u << (vid & 31);
+            is_new = !(atomicOr(vs.bits + (vid >> 5), mask) & mask);
+            if (is_new) {
+                const uint32_t pos = atomicAdd(list_n, 1u);
+                if (pos < vs.list_cap) vs.list[pos] = vid;
+            }
+        }
+    }
+    __syncwarp();
+    return is_new;
+}
+
 __device__ __forceinline__ void table_reset(const Visited& vs) {
     if (vs.tbits) {
         // Two buckets per 16-byte store.
         uint4* t4 = reinterpret_cast<uint4*>(vs.tab);
         const uint32_t n = 1u << (vs.tbits - 1);
+        #pragma unroll 1
         for (uint32_t i = lane_id(); i < n; i += 32) t4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
     }
 }
@@ -690,9 +869,11 @@ __device__ inline void visited_clear(Visited& vs) {
         if (vs.list_overflow) {
             uint4* w4 = reinterpret_cast<uint4*>(vs.bits);
             const uint64_t n4 = vs.words / 4;
+            #pragma unroll 1
             for (uint64_t i = lane; i < n4; i += 32) w4[i] = make_uint4(0, 0, 0, 0);
         } else {
-            for (uint32_t i = lane; i < vs.list_n; i += 32) vs.bits[vs.list[i] >> 5] = 0u;
+            #pragma unroll 4
+            for (uint32_t i = lane; i < vs.list_n; i += 32) vs.bits[__ldcg(vs.list + i) >> 5] = 0u;
         }
         vs.spills++;
     }
@@ -714,6 +895,7 @@ __device__ __forceinline__ void collect_unvisited(const DeviceGraph& g, Visited&
     const int lane = lane_id();
     uint32_t c = 0;
     uint32_t i = start;
+    #pragma unroll 1
     while (i < len && c + 32 <= kCandBatch) {
         const uint32_t idx = i + lane;
         const bool act = idx < len;
@@ -778,6 +960,7 @@ __device__ __forceinline__ uint2 make_ent(float d, uint32_t v) { return make_uin
 __device__ __forceinline__ uint32_t queue_lower_bound(const Queue& q, float d, uint32_t v) {
     const int lane = lane_id();
     uint32_t lo = 0, hi = q.n;
+    #pragma unroll 1
     while (hi - lo > 32) {
         const uint32_t step = (hi - lo + 31) / 32;
         const uint32_t idx = lo + lane * step;
@@ -809,6 +992,7 @@ __device__ __forceinline__ bool queue_insert(Queue& q, float d, uint32_t v, int*
         return false;
     }
     const uint32_t pos = queue_lower_bound(q, d, v);
+    #pragma unroll 1
     for (int end = static_cast<int>(q.n); end > static_cast<int>(pos); end -= 32) {
         const int s = max(static_cast<int>(pos), end - 32);
         const int idx = s + lane;
@@ -827,6 +1011,7 @@ __device__ __forceinline__ bool queue_insert(Queue& q, float d, uint32_t v, int*
         q.lb = ent_d(q.e[q.L - 1]);
         if (q.n > q.L) {
             uint32_t newn = q.n;
+            #pragma unroll 1
             for (uint32_t base = q.L; base < q.n; base += 32) {
                 const uint32_t idx = base + lane;
                 const bool dead = idx < q.n && ent_d(q.e[idx]) > q.lb;
@@ -842,6 +1027,7 @@ __device__ __forceinline__ bool queue_insert(Queue& q, float d, uint32_t v, int*
 // First unexplored entry at or after `from`, or -1.
 __device__ __forceinline__ int queue_find_unexplored(const Queue& q, uint32_t from) {
     const int lane = lane_id();
+    #pragma unroll 1
     for (uint32_t base = from; base < q.n; base += 32) {
         const uint32_t idx = base + lane;
         const bool un = idx < q.n && !(q.e[idx].x & kExplored);
@@ -873,6 +1059,7 @@ __device__ __forceinline__ int queue_pop_peek(Queue& q, int* next) {
     int first = -1;
     *next = -1;
     uint32_t base = q.hint;
+    #pragma unroll 1
     for (; base < q.n; base += 32) {
         const uint32_t idx = base + lane;
         const bool un = idx < q.n && !(q.e[idx].x & kExplored);
@@ -925,6 +1112,7 @@ __device__ inline uint32_t queue_accept(const Queue& q, const uint32_t* cvid, co
     const float lim = q.n >= q.L ? q.lb : INFINITY;
     uint32_t m = 0;
     uint32_t improving_before = 0;   // improving candidates in earlier chunks
+    #pragma unroll 1
     for (uint32_t base = 0; base < cnt; base += 32) {
         const uint32_t j = base + lane;
         const bool valid = j < cnt;
@@ -950,8 +1138,10 @@ __device__ inline uint32_t queue_accept(const Queue& q, const uint32_t* cvid, co
             // shuffles over the improving lanes only.
             uint32_t pre = 0;
             if (improving_before) {
+                #pragma unroll 1
                 for (uint32_t i = 0; i < base; ++i) pre += cdist[i] <= d ? 1u : 0u;
             }
+            #pragma unroll 1
             for (uint32_t bits = imask & lt_mask; __any_sync(kFull, bits != 0);) {
                 // each lane walks its own set of earlier improving lanes; shuffles
                 // need every lane, so lanes take turns through a uniform loop.
@@ -983,6 +1173,7 @@ __device__ inline uint32_t queue_accept(const Queue& q, const uint32_t* cvid, co
 // Number of entries of the sorted array q[0, n) before (d, v) by (dist, vid).
 __device__ __forceinline__ uint32_t old_lower_bound(const Queue& q, float d, uint32_t v) {
     uint32_t lo = 0, hi = q.n;
+    #pragma unroll 1
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
         const uint2 w = q.e[mid];
@@ -1305,6 +1496,24 @@ __device__ __forceinline__ WarpSmem carve(float* base, uint32_t dim, uint32_t ca
     return s;
 }
 
+// The visited set of search slot `slot` (as visited_clear leaves it).
+__device__ __forceinline__ Visited visited_init(const SearchArgs& a, const WarpSmem& sm, uint32_t slot) {
+    Visited vs;
+    vs.tab = reinterpret_cast<uint2*>(sm.vh);
+    vs.tbits = a.vh_bits ? a.vh_bits + 1 : 0u;   // a.vh_bits: log2 of the table's 16-byte units
+    vs.kbits = a.vk_bits;
+    vs.kmask = a.vk_bits >= 32 ? 0xFFFFFFFFu : ((1u << a.vk_bits) - 1u);
+    vs.bits = a.vis_bits + static_cast<size_t>(slot) * a.words_per_slot;
+    vs.list = a.vis_list + static_cast<size_t>(slot) * a.list_cap;
+    vs.list_n = 0;
+    vs.list_cap = a.list_cap;
+    vs.words = a.words_per_slot;
+    vs.global_used = false;
+    vs.list_overflow = false;
+    vs.spills = 0;
+    return vs;
+}
+
 // collect_row64_unique for a fixed-stride row (ids0 = slot lane, ids1 = slot 32 +
 // lane), counting the expansion.
 __device__ __forceinline__ uint32_t collect_pad_row(const DeviceGraph& g, Visited& vs, uint32_t ids0, uint32_t ids1,
@@ -1427,17 +1636,346 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
 }
 
 // ---------------------------------------------------------------------------
+// Level-0 beam search by a team (graphs with fixed-stride rows). The pop order
+// is the pipelined loop's: once the current row's distances are known, the
+// next pop is the smaller of the first unexplored entry and the smallest
+// accepted candidate. One expansion is two barriers: at A the row's distances
+// are written, at B the leader has decided and published the next vertex.
+// Between B and A the row warps expand it (visited test, row loads, distances)
+// while the leader merges the previous row's accepted candidates.
+//
+// A row of 64 slots is cut into kG slices, one per row warp; a warp tests its
+// slice's ids, compacts the new ones to the front of its slice of cvid (slice
+// by slice this is row order) and writes their distances, +inf in the rest of
+// the slice (never accepted). Ids of a row are distinct, so the order in which
+// warps mark them cannot change which are new.
+//
+// A search by one warp is one dependent chain of about 7,000 cycles an
+// expansion on an idle GPU (row ids, visited set, two or three passes of eight
+// rows, acceptance, merge). Here all rows of an expansion are in flight at
+// once and the merge is off the chain; in addition the leader publishes the
+// vertex expected after the next one (the second smallest head), whose ids the
+// row warps load an expansion ahead and whose unvisited rows they start to
+// load before the leader has decided, so on a correct guess (4 of 5) the chain
+// is acceptance, visited test and the rest of the row latency.
+// Against one warp a query: one query of 100k x 128 at queue 64 0.256 -> 0.127 ms,
+// 16 of 200k x 96 cosine at queue 128 0.506 -> 0.262 ms, 256 at queue 100-400 2.20
+// -> 1.16 ms, 1,000 of 100k x 128 at queue 200 1.60 -> 1.09 ms; 10,000 queries are
+// faster with a warp each, which the autotuner finds.
+// ---------------------------------------------------------------------------
+template <int kMetric, bool kExact, int kG>
+__device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem& sm, Visited& vs, int gw, float qsq) {
+    constexpr uint32_t kSlice = kPadRow / kG;
+    static_assert(kSlice <= 32, "one id per lane");
+    const DeviceGraph& g = a.g;
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t lt = (1u << lane) - 1u;
+    CoopCtl* ctl = sm.coop;
+    uint32_t* cv = sm.cvid + gw * kSlice;
+    float* cd = sm.cdist + gw * kSlice;
+    uint32_t* spec = ctl->spec + gw * kSlice;
+    const uint32_t* slice = g.l0pad + gw * kSlice + lane;
+    const bool has = lane < kSlice;
+    const uint32_t pass = (g.dim >> 4) > kBlock ? 2u : 8u;   // rows a pass
+    uint32_t pf_vid = kVidMask, pf_id = 0xffffffffu, spec_mask = 0u;
+    uint32_t evals = 0, row_ids = 0;
+    RowRegs x;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = 0ull;
+    for (;;) {
+        team_wait(kNextBarrier, kG + 1);   // B
+        const uint32_t next = ctl->next;
+        const uint32_t pf = ctl->pf;
+        if (next == kVidMask) break;
+        const bool hit = next == pf_vid;
+        uint32_t id = pf_id;
+        if (!hit) id = has ? __ldg(slice + static_cast<size_t>(next) * kPadRow) : 0xffffffffu;
+        pf_vid = pf;
+        pf_id = (has && pf != kVidMask) ? __ldg(slice + static_cast<size_t>(pf) * kPadRow) : 0xffffffffu;
+        const bool is_new = team_test_and_set(vs, &ctl->list_n, id, id < g.n);
+        const uint32_t b = __ballot_sync(kFull, is_new);
+        const uint32_t cnt = __popc(b);
+        if (is_new) cv[__popc(b & lt)] = id;
+        if (has && lane >= cnt) cd[lane] = INFINITY;
+        __syncwarp();
+        // The rows loaded ahead are the expansion's when the guess was right
+        // and no id was marked in between.
+        if (cnt && !(hit && b == spec_mask)) slice_load(g, cv, 0, cnt, x);
+        #pragma unroll 1
+        for (uint32_t p = 0; p < cnt; p += pass) {
+            if (p) slice_load(g, cv, p, cnt, x);
+            slice_distance<kMetric, kExact>(g, sm.q, qsq, cv, cd, p, cnt, x);
+        }
+        __syncwarp();
+        team_arrive(kRowsBarrier, kG + 1);   // A
+        evals += cnt;
+        row_ids += __popc(__ballot_sync(kFull, id != 0xffffffffu));
+        if (has && id != 0xffffffffu && id >= g.n) set_error(a.error, kErrBadVid);
+        // While the leader decides: the rows of the expected vertex's ids that
+        // are unvisited now.
+        spec_mask = __ballot_sync(kFull, pf_id < g.n && visited_open(vs, pf_id));
+        if (spec_mask) {
+            if ((spec_mask >> lane) & 1u) spec[__popc(spec_mask & lt)] = pf_id;
+            __syncwarp();
+            slice_load(g, spec, 0, __popc(spec_mask), x);
+        }
+    }
+    if (lane == 0) {
+        atomicAdd(&ctl->evals, evals);
+        atomicAdd(&ctl->row_ids, row_ids);
+    }
+    coop_barrier(kG + 1);   // end: counts are in
+}
+
+// Order-preserving unsigned key of a distance (-0 and +0 alike).
+__device__ __forceinline__ uint32_t dist_key(float d) {
+    const uint32_t u = __float_as_uint(d + 0.0f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ bool head_less(uint32_t ka, uint32_t va, uint32_t kb, uint32_t vb) {
+    return ka < kb || (ka == kb && va < vb);
+}
+
+// queue_accept over the 64 slots of cvid/cdist (two a lane), plus the two
+// smallest accepted candidates by (dist, vid): their distance keys and vids
+// (~0u when absent). The candidates stay in registers.
+struct TeamBatch {
+    float d[2];
+    uint32_t v[2];
+    uint32_t acc[2];          // accepted lanes of each half
+    uint32_t m;               // accepted candidates
+    uint32_t k1, v1, k2, v2;
+};
+
+__device__ __forceinline__ void team_accept(const Queue& q, const uint32_t* cvid, const float* cdist, TeamBatch& s) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t tn = min(q.n, q.L);
+    const float lim = q.n >= q.L ? q.lb : INFINITY;
+    s.k1 = s.v1 = s.k2 = s.v2 = 0xffffffffu;
+    s.m = 0;
+    s.d[0] = cdist[lane];
+    s.d[1] = cdist[lane + 32];
+    s.v[0] = cvid[lane];
+    s.v[1] = cvid[lane + 32];
+    s.acc[0] = s.acc[1] = 0u;
+    const uint32_t imp0 = __ballot_sync(kFull, s.d[0] < lim), imp1 = __ballot_sync(kFull, s.d[1] < lim);
+    if ((imp0 | imp1) == 0u) return;   // three of four rows improve nothing
+    // See queue_accept: ub bounds pre, and only lanes it leaves undecided need
+    // the exact count.
+    bool open = false;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const bool improving = s.d[t] < lim;
+        const uint32_t ub = (t ? __popc(imp0) : 0u) + __popc((t ? imp1 : imp0) & lt_mask);
+        bool acc = false;
+        if (improving && ub < q.L) {
+            const uint32_t idx = q.L - ub - 1;
+            acc = idx >= tn || ent_d(q.e[idx]) > s.d[t];
+        }
+        open |= improving && !acc && ub != 0u;
+        s.acc[t] = __ballot_sync(kFull, acc);
+    }
+    if (__any_sync(kFull, open)) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float d = s.d[t];
+            const uint32_t j = lane + 32u * t;
+            uint32_t pre = 0;   // #{i < j : d_i <= d_j}, over the improving candidates
+            #pragma unroll 1
+            for (uint32_t bits = imp0; bits; bits &= bits - 1u) {
+                const uint32_t i = __ffs(bits) - 1u;
+                pre += i < j && cdist[i] <= d ? 1u : 0u;
+            }
+            #pragma unroll 1
+            for (uint32_t bits = t ? imp1 : 0u; bits; bits &= bits - 1u) {
+                const uint32_t i = 32u + __ffs(bits) - 1u;
+                pre += i < j && cdist[i] <= d ? 1u : 0u;
+            }
+            bool acc = false;
+            if (d < lim && pre < q.L) {
+                const uint32_t idx = q.L - pre - 1u;
+                acc = idx >= tn || ent_d(q.e[idx]) > d;
+            }
+            s.acc[t] = __ballot_sync(kFull, acc);
+        }
+    }
+    s.m = __popc(s.acc[0]) + __popc(s.acc[1]);
+    if (s.m == 0u) return;
+    uint32_t key0 = (s.acc[0] >> lane) & 1u ? dist_key(s.d[0]) : 0xffffffffu;
+    uint32_t key1 = (s.acc[1] >> lane) & 1u ? dist_key(s.d[1]) : 0xffffffffu;
+    s.k1 = __reduce_min_sync(kFull, min(key0, key1));
+    s.v1 = __reduce_min_sync(kFull, min(key0 == s.k1 ? s.v[0] : 0xffffffffu, key1 == s.k1 ? s.v[1] : 0xffffffffu));
+    if (s.m > 1u) {
+        if (s.v[0] == s.v1) key0 = 0xffffffffu;
+        if (s.v[1] == s.v1) key1 = 0xffffffffu;
+        s.k2 = __reduce_min_sync(kFull, min(key0, key1));
+        s.v2 = __reduce_min_sync(kFull, min(key0 == s.k2 ? s.v[0] : 0xffffffffu,
+                                            key1 == s.k2 ? s.v[1] : 0xffffffffu));
+    }
+}
+
+// An unexplored entry of the queue: distance key, vid, index (-1: absent).
+struct Head {
+    uint32_t k, v;
+    int at;
+};
+
+__device__ __forceinline__ Head queue_head(const Queue& q, uint32_t from) {
+    const int lane = lane_id();
+    Head h;
+    h.k = h.v = 0xffffffffu;
+    h.at = -1;
+    #pragma unroll 1
+    for (uint32_t base = from; base < q.n; base += 32) {
+        const uint32_t idx = base + lane;
+        const uint2 w = idx < q.n ? q.e[idx] : make_uint2(kExplored, 0u);
+        const uint32_t m = __ballot_sync(kFull, !(w.x & kExplored));
+        if (m) {
+            const int src = __ffs(m) - 1;
+            h.v = __shfl_sync(kFull, w.x, src);
+            h.k = dist_key(__uint_as_float(__shfl_sync(kFull, w.y, src)));
+            h.at = static_cast<int>(base) + src;
+            break;
+        }
+    }
+    return h;
+}
+
+// The leader's side of the level-0 loop. On entry the queue holds the cursor
+// and the cursor is visited. Returns true when the compact queue lost a live
+// entry (see queue_merge).
+template <int kG>
+__device__ __forceinline__ bool l0_team_lead(const SearchArgs& a, Queue& q, Visited& vs, const WarpSmem& sm,
+                                             uint32_t cur, Counters& ct, PhaseClock& pc) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t lt = (1u << lane) - 1u;
+    CoopCtl* ctl = sm.coop;
+    if (lane == 0) {
+        q.e[0].x |= kExplored;   // pop the cursor: the queue's only entry
+        ctl->next = cur;
+        ctl->pf = kVidMask;
+        ctl->list_n = vs.list_overflow ? vs.list_cap + 1u : vs.list_n;
+        ctl->evals = 0;
+        ctl->row_ids = 0;
+        ctl->cmd = kCmdLevel0;
+    }
+    q.hint = 1;
+    coop_barrier(kG + 1);   // start: the row warps enter the loop
+    team_arrive(kNextBarrier, kG + 1);   // B
+    uint32_t m = 0;
+    uint32_t guess = kVidMask;
+    bool lost = false;
+    Head h1, h2;   // the queue's first two unexplored entries
+    h1.k = h1.v = h2.k = h2.v = 0xffffffffu;
+    h1.at = h2.at = -1;
+    for (uint32_t it = 0;; ++it) {
+        ct.l0_rows++;
+        // The previous row's merge runs while this row's distances are computed.
+        if (m) {
+            lost = queue_merge(q, sm.bd, sm.bv, m) && a.compact;
+            h1 = queue_head(q, q.hint);
+            q.hint = h1.at >= 0 ? static_cast<uint32_t>(h1.at) : q.n;
+        }
+        if (h1.at >= 0) h2 = queue_head(q, static_cast<uint32_t>(h1.at) + 1u);
+        pc.lap(kPhMerge);
+        team_wait(kRowsBarrier, kG + 1);   // A: the row's distances are written
+        pc.lap(kPhDist);
+        uint32_t next = kVidMask, pf = kVidMask;
+        bool take_new = false;
+        TeamBatch s;
+        s.m = 0;
+        if (it > a.g.n) {
+            set_error(a.error, kErrBound);
+        } else if (!lost) {
+            team_accept(q, sm.cvid, sm.cdist, s);
+            // Heads: queue (h1, h2) and batch (s.1, s.2), each ascending.
+            take_new = head_less(s.k1, s.v1, h1.k, h1.v);
+            next = take_new ? s.v1 : h1.v;
+            pf = take_new ? (head_less(s.k2, s.v2, h1.k, h1.v) ? s.v2 : h1.v)
+                          : (head_less(s.k1, s.v1, h2.k, h2.v) ? s.v1 : h2.v);
+            next &= kVidMask;   // absent: kVidMask
+            pf &= kVidMask;
+        }
+        if (lane == 0) {
+            ctl->next = next;
+            ctl->pf = pf;
+        }
+        __syncwarp();
+        team_arrive(kNextBarrier, kG + 1);   // B
+        if (next == kVidMask) break;
+        // Off the row warps' chain: the accepted candidates, in slot order, to
+        // bd/bv for the merge; the popped entry marked explored where it lies.
+        m = s.m;
+        if (m) {
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                if ((s.acc[t] >> lane) & 1u) {
+                    const uint32_t k = (t ? __popc(s.acc[0]) : 0u) + __popc(s.acc[t] & lt);
+                    sm.bd[k] = s.d[t];
+                    sm.bv[k] = s.v[t] | (take_new && s.v[t] == s.v1 ? kExplored : 0u);
+                }
+            }
+        }
+        if (!take_new) {
+            if (lane == 0) q.e[h1.at].x |= kExplored;
+            q.hint = static_cast<uint32_t>(h1.at) + 1u;
+            h1 = h2;   // (a merge finds both anew)
+            h2.k = h2.v = 0xffffffffu;
+            h2.at = -1;
+        }
+        __syncwarp();
+        if (next == guess) pc.count(kPhPrefetchHits);
+        guess = pf;
+        pc.lap(kPhPop);
+    }
+    coop_barrier(kG + 1);   // end: counts are in
+    const uint32_t list_n = ctl->list_n;
+    vs.global_used = list_n != 0u;
+    vs.list_overflow = list_n > vs.list_cap;
+    vs.list_n = min(list_n, vs.list_cap);
+    ct.dist_evals += ctl->evals;
+    ct.l0_row_ids += ctl->row_ids;
+    return lost;
+}
+
+// The row warps of a team: follow the leader's commands until it quits.
+template <int kMetric, bool kExact, int kG, bool kPad>
+__device__ void team_rows(const SearchArgs& a, const WarpSmem& sm, int warp) {
+    CoopCtl* ctl = sm.coop;
+    Stage st;
+    st.buf = nullptr;
+    st.mbar = 0u;
+    st.phase = 0u;
+    Visited vs = visited_init(a, sm, blockIdx.x);
+    for (;;) {
+        coop_barrier(kG + 1);   // start
+        const uint32_t cmd = ctl->cmd;
+        const float qsq = ctl->qsq;
+        if (cmd == kCmdQuit) break;
+        if (kPad && cmd == kCmdLevel0) {
+            l0_team_rows<kMetric, kExact, kG>(a, sm, vs, warp - 1, qsq);
+            continue;
+        }
+        batch_distances<kMetric, kExact, false, false, true>(a.g, sm.q, qsq, ctl->cvid, ctl->cdist, ctl->cnt, st,
+                                                            a.error, nullptr, static_cast<uint32_t>(warp), kG + 1);
+        coop_barrier(kG + 1);   // done
+    }
+}
+
+// ---------------------------------------------------------------------------
 // One query (hierarchical_graph_router.hpp:195-248; query_l0_only :258-286).
 // ---------------------------------------------------------------------------
 // stage_phase: with kStage, the parity of the next phase of the warp's staging
 // mbarrier, which the caller initialised once (an mbarrier is not initialised
 // again while it is valid) and which carries over from query to query.
-// kPipe: the kernel carries the pipelined level-0 loop (taken when a.l0_pipe;
-// otherwise, and in kernels without it, one expansion at a time). kRegs: the
+// kPipe: level 0 by the pipelined loop, or the team's (fixed-stride rows), else
+// one expansion at a time. kRegs: the
 // pipelined loop holds the next expansion's first pass in registers (the
-// 128-register budget) instead of prefetching it into L2. kW: warps per query.
+// 128-register budget) instead of prefetching it into L2. kG: row warps of a team
+// whose leader runs this (0: one warp searches alone).
 // kTrace: record the search in a.tr (the probes' trace kernel).
-template <int kMetric, bool kExact, bool kStage = false, bool kRegs = false, int kW = 1, bool kPipe = false,
+template <int kMetric, bool kExact, bool kStage = false, bool kRegs = false, int kG = 0, bool kPipe = false,
           bool kTrace = false>
 __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, const WarpSmem& sm,
                            uint32_t* stage_phase = nullptr) {
@@ -1451,6 +1989,7 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
 
     if (topk > a.k_stride || L < topk || (a.compact ? L + 1ull : 2ull * L) > a.cap) {
         set_error(a.error, kErrArgs);
+        #pragma unroll 1
         for (uint32_t i = lane; i < a.k_stride; i += 32) out[i] = kInvalidWord;
         return;
     }
@@ -1461,19 +2000,7 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
     PhaseClock pc;
     pc.start(a.phase_cycles != nullptr, sm.phase);
     const long long t_begin = pc.on ? clock64() : 0;
-    Visited vs;
-    vs.tab = reinterpret_cast<uint2*>(sm.vh);
-    vs.tbits = a.vh_bits ? a.vh_bits + 1 : 0u;   // a.vh_bits: log2 of the table's 16-byte units
-    vs.kbits = a.vk_bits;
-    vs.kmask = a.vk_bits >= 32 ? 0xFFFFFFFFu : ((1u << a.vk_bits) - 1u);
-    vs.bits = a.vis_bits + static_cast<size_t>(slot) * a.words_per_slot;
-    vs.list = a.vis_list + static_cast<size_t>(slot) * a.list_cap;
-    vs.list_n = 0;
-    vs.list_cap = a.list_cap;
-    vs.words = a.words_per_slot;
-    vs.global_used = false;
-    vs.list_overflow = false;
-    vs.spills = 0;
+    Visited vs = visited_init(a, sm, slot);
     uint32_t* cvid = sm.cvid;
     float* cdist = sm.cdist;
     Stage st;
@@ -1485,85 +2012,108 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
         // Stage the query row in shared memory; reset the visited hash.
         const float4* src = reinterpret_cast<const float4*>(a.queries + static_cast<size_t>(qi) * dim);
         float4* dst = reinterpret_cast<float4*>(sm.q);
+        #pragma unroll 1
         for (uint32_t i = lane; i < dim / 4; i += 32) dst[i] = a.coherent ? __ldcg(src + i) : __ldg(src + i);
         table_reset(vs);
         __syncwarp();
         const float qsq = (kMetric == ARTEA_GPU_COSINE) ? query_sqnorm<kExact>(sm.q, dim) : 0.f;
 
-        // Entry point distance (hierarchical_graph_router.hpp:209-211).
+        // Entry point distance (hierarchical_graph_router.hpp:209-211), then the
+        // greedy descent, levels top..1 (:228-236): one loop with one distance
+        // call and one visited test for all of it, so that its code stays small.
         uint32_t cur = g.entry;
+        float cur_d = 0.0f, best_d = 0.0f;
+        uint32_t best_v = cur;
+        uint32_t h = (a.l0_only ? 0u : g.top) + 1u;   // level walked (one above: the entry point is evaluated)
+        const uint32_t h_top = h;
+        const uint32_t* row = nullptr;
+        uint32_t len = 0, pos = 0, hop = 0, cnt = 1;
         if (lane == 0) cvid[0] = cur;
         __syncwarp();
-        dist_call<kMetric, kExact, kStage, kW>(g, sm.q, qsq, cvid, cdist, 1, st, a.error, sm.coop);
-        float cur_d = cdist[0];
-        ct.dist_evals = 1;
-
-        // Greedy descent, levels top..1 (hierarchical_graph_router.hpp:228-236).
-        if (!a.l0_only) {
-            for (uint32_t h = g.top; h >= 1; --h) {
-                visited_set(vs, cur);
-                for (uint32_t hop = 0;; ++hop) {
-                    if (hop > g.n) { set_error(a.error, kErrBound); break; }
-                    // enable_early_stop: detail/beam_loop.hpp:147-150.
-                    if (a.early_stop && cur_d <= a.es_thr[h]) break;
-                    uint32_t len;
-                    const uint32_t* row = level_row(g, cur, h, &len);
-                    ct.upper_rows++;
-                    ct.upper_row_ids += len;
-                    float best_d = cur_d;
-                    uint32_t best_v = cur;
-                    uint32_t pos = 0;
-                    while (pos < len) {
-                        uint32_t cnt, consumed;
-                        collect_unvisited(g, vs, row, len, pos, cvid, &cnt, &consumed, a.error, 0u, 0u, false);
-                        pos = consumed;
-                        if (cnt == 0) continue;
-                        dist_call<kMetric, kExact, kStage, kW>(g, sm.q, qsq, cvid, cdist, cnt, st, a.error,
-                                                               sm.coop);
-                        ct.dist_evals += cnt;
-                        ct.upper_dist_evals += cnt;
-                        // First strict improvement in row order (beam_loop.hpp:153-160).
-                        float md = INFINITY;
-                        uint32_t mi = 0xffffffffu;
-                        for (uint32_t i = lane; i < cnt; i += 32) {
-                            const float d = cdist[i];
-                            if (d < md) { md = d; mi = i; }
-                        }
-                        for (int off = 16; off > 0; off >>= 1) {
-                            const float od = __shfl_xor_sync(kFull, md, off);
-                            const uint32_t oi = __shfl_xor_sync(kFull, mi, off);
-                            if (od < md || (od == md && oi < mi)) { md = od; mi = oi; }
-                        }
-                        if (md < best_d) {
-                            best_d = md;
-                            best_v = cvid[mi];
-                        }
-                        __syncwarp();
+        #pragma unroll 1
+        for (;;) {
+            if (cnt) {
+                dist_call<kMetric, kExact, kStage, kG>(g, sm.q, qsq, cvid, cdist, cnt, st, a.error, sm.coop);
+                ct.dist_evals += cnt;
+                if (h == h_top) {
+                    cur_d = cdist[0];
+                } else {
+                    ct.upper_dist_evals += cnt;
+                    // First strict improvement in row order (beam_loop.hpp:153-160).
+                    float md = INFINITY;
+                    uint32_t mi = 0xffffffffu;
+                    #pragma unroll 1
+                    for (uint32_t i = lane; i < cnt; i += 32) {
+                        const float d = cdist[i];
+                        if (d < md) { md = d; mi = i; }
                     }
-                    if (best_v == cur) break;
-                    cur = best_v;
-                    cur_d = best_d;
+                    #pragma unroll 1
+                    for (int off = 16; off > 0; off >>= 1) {
+                        const float od = __shfl_xor_sync(kFull, md, off);
+                        const uint32_t oi = __shfl_xor_sync(kFull, mi, off);
+                        if (od < md || (od == md && oi < mi)) { md = od; mi = oi; }
+                    }
+                    if (md < best_d) {
+                        best_d = md;
+                        best_v = cvid[mi];
+                    }
+                    __syncwarp();
                 }
-                visited_clear(vs);
+                cnt = 0;
             }
+            if (pos < len) {
+                uint32_t consumed;
+                collect_unvisited(g, vs, row, len, pos, cvid, &cnt, &consumed, a.error, 0u, 0u, false);
+                pos = consumed;
+                continue;
+            }
+            // The row is done: walk on, or end the level.
+            bool ends = h == h_top || best_v == cur;
+            if (!ends) {
+                cur = best_v;
+                cur_d = best_d;
+                if (++hop > g.n) { set_error(a.error, kErrBound); ends = true; }
+            }
+            // enable_early_stop: detail/beam_loop.hpp:147-150.
+            if (!ends && a.early_stop && cur_d <= a.es_thr[h]) ends = true;
+            if (ends) {
+                if (h != h_top) visited_clear(vs);
+                bool stop;
+                do {
+                    --h;
+                    hop = 0;
+                    visited_set(vs, cur);
+                    stop = h != 0u && a.early_stop && cur_d <= a.es_thr[h];
+                    if (stop) visited_clear(vs);
+                } while (stop);
+                if (h == 0u) break;
+            }
+            row = level_row(g, cur, h, &len);
+            pos = 0;
+            best_d = cur_d;
+            best_v = cur;
+            ct.upper_rows++;
+            ct.upper_row_ids += len;
         }
         pc.lap(kPhUpper);
 
         // Level-0 beam search (single_layer_router.hpp:145-163, beam_loop.hpp:90-119).
         Queue q;
         q.e = sm.qe;
-        q.n = 0;
+        q.n = 1;
         q.L = L;
         q.cap = a.cap;
         q.hint = 0;
-        q.lb = FLT_MAX;
-        queue_insert(q, cur_d, cur, a.error);
-        visited_set(vs, cur);
+        q.lb = L == 1u ? cur_d : FLT_MAX;
+        if (lane == 0) q.e[0] = make_ent(cur_d, cur);
+        __syncwarp();
         uint32_t tpos = 0, trows = 0;   // kTrace: candidates and rows recorded
         if (kTrace && lane == 0) a.tr.cur[qi] = make_uint2(cur, __float_as_uint(cur_d));
         if (kTrace && a.tr.upper_only) {
             // The greedy descent alone: level 0 is not searched.
-        } else if (kPipe && !kStage && kW == 1 && a.l0_pipe) {
+        } else if (kG > 0 && kPipe) {
+            overflowed = l0_team_lead<kG>(a, q, vs, sm, cur, ct, pc) && a.compact;
+        } else if (kPipe) {
             overflowed = l0_search_pipelined<kMetric, kExact, kRegs>(a, q, vs, sm, qsq, cur, ct, pc, st) &&
                          a.compact;
         } else {
@@ -1574,6 +2124,7 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
             unsigned long long pf_desc = __ldg(g.l0row + cur);
             uint32_t pf_ids0 = 0u, pf_ids1 = 0u;
             bool pf_have_ids = false;
+            #pragma unroll 1
             for (uint32_t it = 0;; ++it) {
                 if (it > g.n) { set_error(a.error, kErrBound); break; }
                 int p2;
@@ -1606,6 +2157,7 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
                 pc.lap(kPhPop);
                 uint32_t pos = 0;
                 const bool one_pass = g.l0_unique && len <= 64u;
+                #pragma unroll 1
                 while (pos < len) {
                     uint32_t cnt, consumed;
                     if (one_pass) {
@@ -1622,9 +2174,10 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
                         ++trows;
                     }
                     if (cnt == 0) continue;
-                    dist_call<kMetric, kExact, kStage, kW>(g, sm.q, qsq, cvid, cdist, cnt, st, a.error, sm.coop);
+                    dist_call<kMetric, kExact, kStage, kG>(g, sm.q, qsq, cvid, cdist, cnt, st, a.error, sm.coop);
                     ct.dist_evals += cnt;
                     if (kTrace) {
+                        #pragma unroll 1
                         for (uint32_t i = lane; i < cnt; i += 32) {
                             if (tpos + i < a.tr.cap) {
                                 a.tr.ids[static_cast<size_t>(qi) * a.tr.cap + tpos + i] = cvid[i];
@@ -1669,6 +2222,7 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
         // extract_results(min(topk, |T|)) (std_candidate_queue.hpp:542-561).
         const uint32_t tsize = min(q.n, q.L);
         nres = min(topk, tsize);
+        #pragma unroll 1
         for (uint32_t i = lane; i < a.k_stride; i += 32) {
             uint64_t w = kInvalidWord;
             if (i < nres) {
@@ -1678,6 +2232,7 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
             out[i] = w;
         }
     } else {
+        #pragma unroll 1
         for (uint32_t i = lane; i < a.k_stride; i += 32) out[i] = kInvalidWord;
     }
 
@@ -1711,7 +2266,7 @@ __global__ void __launch_bounds__(32, 24) search_plain_kernel(SearchArgs a) {
     const uint32_t qi = blockIdx.x;
     if (qi >= a.nq) return;
     const WarpSmem sm = carve(smem, a.g.dim, a.cap);
-    search_one<kMetric, kExact, false, false, 1, kPipe>(a, qi, qi, sm);
+    search_one<kMetric, kExact, false, false, 0, kPipe>(a, qi, qi, sm);
 }
 
 // Persistent schedule: warps pull query indices from a shared counter (in
@@ -1747,7 +2302,7 @@ __global__ void __launch_bounds__(budget_threads(kBudget), budget_min_blocks(kBu
         qi = __shfl_sync(kFull, qi, 0);
         if (qi >= a.nq) break;
         if (a.order) qi = __ldg(a.order + qi);
-        search_one<kMetric, kExact, kStage, kBudget == 128, 1, kPipe>(a, qi, slot, sm, &stage_phase);
+        search_one<kMetric, kExact, kStage, kBudget == 128, 0, kPipe>(a, qi, slot, sm, &stage_phase);
     }
     if (kStage) {
         __syncwarp();
@@ -1772,21 +2327,23 @@ __global__ void __launch_bounds__(32, 24) search_rerun_kernel(SearchArgs a) {
     }
 }
 
-// Cooperative persistent schedule: a CTA of kW warps searches one query at a
-// time (queries from the shared counter, in a.order if set); warp 0 runs the
-// search, and every distance batch is split over the kW warps (CoopCtl).
-// Launch bounds give each thread 96 registers. Rows are read with vector
-// loads; the level-0 loop takes one expansion at a time.
-template <int kMetric, bool kExact, int kW>
-__global__ void __launch_bounds__(kW * 32, 20 / kW) search_coop_kernel(SearchArgs a) {
+// Team schedule: a CTA of kG row warps and a leader searches one query at a
+// time (queries from the shared counter, in a.order if set). Rows are read with
+// vector loads. Launch bounds leave at least 96 registers a thread: the row
+// warps hold the expected expansion's first rows in registers.
+constexpr int team_min_blocks(int g) { return g == 2 ? 6 : (g == 4 ? 4 : 2); }
+
+// kPad: level 0 split over the team (fixed-stride rows); else one expansion at a
+// time by the leader, its distance batches split over the warps.
+template <int kMetric, bool kExact, int kG, bool kPad>
+__global__ void __launch_bounds__((kG + 1) * 32, team_min_blocks(kG)) search_team_kernel(SearchArgs a) {
     extern __shared__ __align__(16) float smem[];
     const int warp = threadIdx.x >> 5;
     const uint32_t words = warp_smem_words(a.g.dim, a.cap, a.vh_bits);
     WarpSmem sm = carve(smem, a.g.dim, a.cap);
-    CoopCtl* coop = reinterpret_cast<CoopCtl*>(smem + words);
-    sm.coop = coop;
+    sm.coop = reinterpret_cast<CoopCtl*>(smem + words);
     if (warp != 0) {
-        coop_helper<kMetric, kExact, kW>(a.g, sm.q, coop, warp, a.error);
+        team_rows<kMetric, kExact, kG, kPad>(a, sm, warp);
         return;
     }
     for (;;) {
@@ -1795,10 +2352,10 @@ __global__ void __launch_bounds__(kW * 32, 20 / kW) search_coop_kernel(SearchArg
         qi = __shfl_sync(kFull, qi, 0);
         if (qi >= a.nq) break;
         if (a.order) qi = __ldg(a.order + qi);
-        search_one<kMetric, kExact, false, false, kW>(a, qi, blockIdx.x, sm);
+        search_one<kMetric, kExact, false, false, kG, kPad>(a, qi, blockIdx.x, sm);
     }
-    if (lane_id() == 0) coop->quit = 1u;
-    coop_barrier(kW);   // the helpers see quit and leave
+    if (lane_id() == 0) sm.coop->cmd = kCmdQuit;
+    coop_barrier(kG + 1);   // the row warps see quit and leave
 }
 
 }  // namespace artea_gpu

@@ -175,12 +175,12 @@ typedef struct artea_gpu_router_opts {
                                    queries fill the tail), 0xFFFFFFFF = index
                                    order. Results do not depend on it. */
     uint32_t warps_per_query;   /* persistent schedule: 1 = one warp searches a
-                                   query; 2 or 4 = a CTA of that many warps
-                                   searches one query, its distance batches
-                                   split over the warps (for few, long
-                                   searches: small batches, large dims);
-                                   0 = autotuned */
-    uint32_t queue_slack;       /* persistent one-warp kernels' queue layout:
+                                   query; 2 or 4 = a CTA searches one query, a
+                                   small team (2 or 4 warps reading rows and one
+                                   keeping the queue) or a large one (8 and
+                                   one), for batches that leave the GPU idle
+                                   and large dims; 0 = autotuned */
+    uint32_t queue_slack;       /* persistent kernels' queue layout:
                                    0xFFFFFFFF = 2L entries per search (room for
                                    every tie of lb the reference keeps);
                                    1..4096 = compact, max queue + that many
