@@ -17,6 +17,7 @@
 #include <cstdlib>
 
 #include "../../include/artea_gpu.h"
+#include "bruteforce.h"
 #include "common.h"
 #include "internal.h"
 #include "search.cuh"
@@ -1005,7 +1006,9 @@ int index_begin(uint32_t num_vertices, const float* vectors, uint32_t num_vector
             artea_gpu_index_destroy(ix);
             return fail(ARTEA_GPU_ECUDA, "row norms failed");
         }
+        ix->bf = bf_cache_create(ix->d_xsq, num_vectors, std::max(sms, 1));
     }
+    if (!ix->bf) ix->bf = bf_cache_create(nullptr, 0, 1);
     *out = ix;
     return ARTEA_GPU_OK;
 }
@@ -1135,6 +1138,7 @@ int artea_gpu_index_destroy(artea_gpu_index* ix) {
     dev_free(ix->d_offsets);
     dev_free(ix->d_l0row);
     dev_free(ix->d_l0pad);
+    bf_cache_destroy(ix->bf);
     delete ix;
     return ARTEA_GPU_OK;
 }

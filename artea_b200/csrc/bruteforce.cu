@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/artea_gpu.h"
+#include "bruteforce.h"
 #include "common.h"
 #include "internal.h"
 
@@ -29,6 +30,8 @@ namespace {
 constexpr int kBfQueries = 8;        // queries per CTA
 constexpr int kBfThreads = 128;      // rows per round (one per thread)
 constexpr uint32_t kBfMaxTopk = 1024;
+constexpr uint32_t kFilterRows = 8192;   // fewer rows: the scan
+constexpr uint32_t kFilterQueries = 16;  // fewer queries: the scan, unless the index's rows are rounded already
 constexpr uint64_t kMaxKey = ~0ull;
 // CandidateEntry() (router/data_structures/candidate_entry.hpp:72-74): vid =
 // invalid_vertex_id (all ones), distance 0 -- the padding of batch rows whose
@@ -321,27 +324,10 @@ ScanFn scan_kernel(int metric) {
     }
 }
 
-// use_subset: rows are d_subset[0, n_subset) (possibly empty), else all vectors.
-int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
-                    bool use_subset, const uint32_t* d_subset, uint32_t n_subset, uint64_t* d_out, cudaStream_t st) {
-    if (!ix || (nq && (!d_queries || !d_out))) return fail(ARTEA_GPU_EINVAL, "null argument");
-    if (topk == 0 || topk > kBfMaxTopk)
-        return fail(ARTEA_GPU_EINVAL, "brute-force topk must be in [1, " + std::to_string(kBfMaxTopk) + "]");
+// The FP32 scan of rows [0, n_rows) (d_subset null) or d_subset's; waits.
+int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
+         const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int dev_sms, cudaStream_t st) {
     ScanFn fn = scan_kernel(metric);
-    if (!fn) return fail(ARTEA_GPU_EINVAL, "unknown metric");
-    if (nq == 0) return ARTEA_GPU_OK;
-    const uint32_t n_rows = use_subset ? n_subset : ix->nvecs;
-    if (use_subset && n_subset && !d_subset) return fail(ARTEA_GPU_EINVAL, "null subset");
-    DeviceGuard guard(ix->device);
-    if (n_rows == 0) {
-        // Every row is CandidateEntry() padding.
-        std::vector<uint64_t> pad(static_cast<size_t>(nq) * topk, kDefaultEntryWord);
-        CUDA_TRY(cudaMemcpyAsync(d_out, pad.data(), pad.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        return ARTEA_GPU_OK;
-    }
-    int dev_sms = 0;
-    CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ix->device));
     const uint32_t list_cap = next_pow2(topk + 2 * kBfThreads);
     const size_t smem = static_cast<size_t>(kBfQueries) * list_cap * sizeof(uint64_t) +
                         static_cast<size_t>(kBfQueries) * ix->dim * sizeof(float);
@@ -365,7 +351,7 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
     std::memset(&a, 0, sizeof(a));
     a.vecs = ix->d_vecs;
     a.dim = ix->dim;
-    a.subset = use_subset ? d_subset : nullptr;
+    a.subset = d_subset;
     a.n_rows = n_rows;
     a.queries = d_queries;
     a.nq = nq;
@@ -374,16 +360,12 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
     a.segments = segments;
     a.list_cap = list_cap;
     a.out = d_out;
-    uint64_t* part = nullptr;
-    uint32_t* part_n = nullptr;
     if (segments > 1) {
-        if (int rc = dev_alloc(&part, static_cast<size_t>(nq) * segments * topk)) return rc;
-        if (int rc = dev_alloc(&part_n, static_cast<size_t>(nq) * segments)) {
-            dev_free(part);
-            return rc;
-        }
-        a.part = part;
-        a.part_n = part_n;
+        const size_t keys = sizeof(uint64_t) * static_cast<size_t>(nq) * segments * topk;
+        unsigned char* p = nullptr;
+        if (int rc = work.get(1, keys + sizeof(uint32_t) * static_cast<size_t>(nq) * segments, &p)) return rc;
+        a.part = reinterpret_cast<uint64_t*>(p);
+        a.part_n = reinterpret_cast<uint32_t*>(p + keys);
     }
     fn<<<dim3(tiles, segments), kBfThreads, smem, st>>>(a);
     cudaError_t e = cudaGetLastError();
@@ -393,15 +375,56 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(bf_merge_kernel),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(msmem));
         if (e == cudaSuccess) {
-            bf_merge_kernel<<<nq, 256, msmem, st>>>(part, part_n, segments, topk, pow2, d_out);
+            bf_merge_kernel<<<nq, 256, msmem, st>>>(a.part, a.part_n, segments, topk, pow2, d_out);
             e = cudaGetLastError();
         }
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    dev_free(part);
-    dev_free(part_n);
     if (e != cudaSuccess) return fail(ARTEA_GPU_ECUDA, std::string("brute force: ") + cudaGetErrorString(e));
     return ARTEA_GPU_OK;
+}
+
+// use_subset: rows are d_subset[0, n_subset) (possibly empty), else all vectors.
+int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
+                    bool use_subset, const uint32_t* d_subset, uint32_t n_subset, uint64_t* d_out, BfWork& work,
+                    cudaStream_t st) {
+    if (!ix || (nq && (!d_queries || !d_out))) return fail(ARTEA_GPU_EINVAL, "null argument");
+    if (topk == 0 || topk > kBfMaxTopk)
+        return fail(ARTEA_GPU_EINVAL, "brute-force topk must be in [1, " + std::to_string(kBfMaxTopk) + "]");
+    if (!scan_kernel(metric)) return fail(ARTEA_GPU_EINVAL, "unknown metric");
+    if (nq == 0) return ARTEA_GPU_OK;
+    const uint32_t n_rows = use_subset ? n_subset : ix->nvecs;
+    if (use_subset && n_subset && !d_subset) return fail(ARTEA_GPU_EINVAL, "null subset");
+    DeviceGuard guard(ix->device);
+    if (n_rows == 0) {
+        // Every row is CandidateEntry() padding.
+        std::vector<uint64_t> pad(static_cast<size_t>(nq) * topk, kDefaultEntryWord);
+        CUDA_TRY(cudaMemcpyAsync(d_out, pad.data(), pad.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        return ARTEA_GPU_OK;
+    }
+    int dev_sms = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ix->device));
+    const uint32_t* subset = use_subset ? d_subset : nullptr;
+    // The tensor-core filter reads every row twice in FP16 and pays a rounding pass
+    // over the rows (once an index, or on every call for a subset); the scan reads
+    // them once in FP32 for every 8 queries. With fewer rows the launches decide.
+    const bool filter = n_rows >= kFilterRows && 8ull * topk <= n_rows &&
+                        (nq >= kFilterQueries || (!use_subset && bf_rows_ready(ix)));
+    if (filter) {
+        bool used = false;
+        std::vector<uint32_t> redo;
+        if (int rc = bf_tensor(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &used, &redo))
+            return rc;
+        if (used && redo.size() <= 64) {
+            for (const uint32_t q : redo)
+                if (int rc = scan(ix, metric, d_queries + static_cast<size_t>(q) * ix->dim, 1, topk, subset, n_rows,
+                                  d_out + static_cast<size_t>(q) * topk, work, dev_sms, st))
+                    return rc;
+            return ARTEA_GPU_OK;
+        }
+    }
+    return scan(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st);
 }
 
 // Centroid of the bucket's rows (hierarchical_graph_compactor.hpp:261-300):
@@ -442,7 +465,10 @@ extern "C" {
 int artea_gpu_bruteforce_device(const artea_gpu_index* index, int metric, const float* d_queries, uint32_t nq,
                                 uint32_t topk, const uint32_t* d_subset, uint32_t n_subset, uint64_t* d_out,
                                 void* stream) {
-    return bruteforce_impl(index, metric, d_queries, nq, topk, d_subset != nullptr, d_subset, n_subset, d_out,
+    if (!index) return fail(ARTEA_GPU_EINVAL, "null argument");
+    DeviceGuard guard(index->device);
+    BfWork work(index);
+    return bruteforce_impl(index, metric, d_queries, nq, topk, d_subset != nullptr, d_subset, n_subset, d_out, work,
                            static_cast<cudaStream_t>(stream));
 }
 
@@ -456,24 +482,24 @@ int artea_gpu_bruteforce(const artea_gpu_index* index, int metric, const float* 
     }
     if (nq == 0) return ARTEA_GPU_OK;
     DeviceGuard guard(index->device);
-    float* d_q = nullptr;
-    uint64_t* d_o = nullptr;
-    uint32_t* d_s = nullptr;
-    int rc = dev_alloc(&d_q, static_cast<size_t>(nq) * index->dim);
-    if (!rc) rc = dev_alloc(&d_o, static_cast<size_t>(nq) * topk);
-    if (!rc && subset && n_subset) rc = dev_alloc(&d_s, n_subset);
-    if (!rc && cudaMemcpy(d_q, queries, sizeof(float) * nq * index->dim, cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = fail(ARTEA_GPU_ECUDA, "query upload failed");
-    if (!rc && d_s && cudaMemcpy(d_s, subset, sizeof(uint32_t) * n_subset, cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = fail(ARTEA_GPU_ECUDA, "subset upload failed");
-    if (!rc) rc = bruteforce_impl(index, metric, d_q, nq, topk, subset != nullptr, d_s, subset ? n_subset : 0u, d_o,
-                                  nullptr);
-    if (!rc && cudaMemcpy(out, d_o, sizeof(uint64_t) * nq * topk, cudaMemcpyDeviceToHost) != cudaSuccess)
-        rc = fail(ARTEA_GPU_ECUDA, "result download failed");
-    dev_free(d_q);
-    dev_free(d_o);
-    dev_free(d_s);
-    return rc;
+    BfWork work(index);
+    const size_t q_bytes = (sizeof(float) * nq * index->dim + 255) / 256 * 256;
+    const size_t o_bytes = (sizeof(uint64_t) * nq * static_cast<size_t>(topk) + 255) / 256 * 256;
+    unsigned char* p = nullptr;
+    if (int rc = work.get(0, q_bytes + o_bytes + (subset ? sizeof(uint32_t) * n_subset : 0) + 1, &p)) return rc;
+    float* d_q = reinterpret_cast<float*>(p);
+    uint64_t* d_o = reinterpret_cast<uint64_t*>(p + q_bytes);
+    uint32_t* d_s = subset && n_subset ? reinterpret_cast<uint32_t*>(p + q_bytes + o_bytes) : nullptr;
+    if (cudaMemcpy(d_q, queries, sizeof(float) * nq * index->dim, cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(ARTEA_GPU_ECUDA, "query upload failed");
+    if (d_s && cudaMemcpy(d_s, subset, sizeof(uint32_t) * n_subset, cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(ARTEA_GPU_ECUDA, "subset upload failed");
+    if (int rc = bruteforce_impl(index, metric, d_q, nq, topk, subset != nullptr, d_s, subset ? n_subset : 0u, d_o, work,
+                                 nullptr))
+        return rc;
+    if (cudaMemcpy(out, d_o, sizeof(uint64_t) * nq * topk, cudaMemcpyDeviceToHost) != cudaSuccess)
+        return fail(ARTEA_GPU_ECUDA, "result download failed");
+    return ARTEA_GPU_OK;
 }
 
 // _compute_entry_point_vid (hierarchical_graph_compactor.hpp:261-327): the
@@ -511,7 +537,10 @@ int artea_gpu_centroid_entry(const artea_gpu_index* index, int metric, const uin
         centroid_final_kernel<<<(index->dim + 255) / 256, 256>>>(d_partial, blocks, index->dim, rows, d_centroid);
         if (cudaGetLastError() != cudaSuccess) rc = fail(ARTEA_GPU_ECUDA, "centroid kernels failed to launch");
     }
-    if (!rc) rc = bruteforce_impl(index, metric, d_centroid, 1, 1, bucket != nullptr, d_bucket, rows, d_word, nullptr);
+    if (!rc) {
+        BfWork work(index);
+        rc = bruteforce_impl(index, metric, d_centroid, 1, 1, bucket != nullptr, d_bucket, rows, d_word, work, nullptr);
+    }
     uint64_t word = 0;
     if (!rc && cudaMemcpy(&word, d_word, sizeof(word), cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = fail(ARTEA_GPU_ECUDA, "result download failed");

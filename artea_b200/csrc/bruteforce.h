@@ -1,0 +1,44 @@
+// Brute force through the tensor cores (bruteforce_tc.cu), used by bruteforce.cu.
+#pragma once
+
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+struct artea_gpu_index;
+
+namespace artea_gpu {
+
+struct BfCache;
+BfCache* bf_cache_create(const float* d_xsq, uint32_t n, int sms);   // x.x of every row
+void bf_cache_destroy(BfCache* c);
+
+// A call's device workspace: the index's, unless another thread's call holds it.
+// Slot 0: the host entry points' copies; slot 1: everything else.
+constexpr size_t kBfKeepBytes = 256u << 20;   // the index keeps no larger one
+struct BfWork {
+    explicit BfWork(const artea_gpu_index* ix);
+    ~BfWork();
+    BfWork(const BfWork&) = delete;
+    BfWork& operator=(const BfWork&) = delete;
+    // At least bytes, valid until the slot's next get() or the end.
+    int get(int slot, size_t bytes, unsigned char** p);
+
+    BfCache* cache;
+    bool held = false;
+    unsigned char* own[2] = {};
+};
+
+// Whether the index holds its rounded rows already.
+bool bf_rows_ready(const artea_gpu_index* ix);
+
+// Ranks rows [0, n_rows) (or those of d_subset) for nq queries into d_out, and waits.
+// *used false: nothing was written (the filter does not apply). redo: queries left
+// to the scan.
+int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
+              const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int sms, cudaStream_t st,
+              bool* used, std::vector<uint32_t>* redo);
+
+}  // namespace artea_gpu

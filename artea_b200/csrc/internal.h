@@ -19,6 +19,10 @@ using artea_gpu::fail;
         if (_e != cudaSuccess) return fail(ARTEA_GPU_ECUDA, std::string(#expr) + ": " + cudaGetErrorString(_e)); \
     } while (0)
 
+namespace artea_gpu {
+struct BfCache;
+}
+
 // A device-resident graph plus its vectors (artea_gpu_index_create).
 struct artea_gpu_index {
     int device = 0;
@@ -36,6 +40,7 @@ struct artea_gpu_index {
     uint64_t n_offsets = 0;   // entries of d_offsets (all groups, with their end sentinels)
     uint64_t n_nbrs = 0;      // entries of d_nbrs in use
     uint64_t bytes = 0;
+    artea_gpu::BfCache* bf = nullptr;   // brute force: rounded rows, workspace (bruteforce_tc.cu)
 };
 
 namespace artea_gpu {
