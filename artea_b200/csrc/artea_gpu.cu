@@ -1006,9 +1006,9 @@ int index_begin(uint32_t num_vertices, const float* vectors, uint32_t num_vector
             artea_gpu_index_destroy(ix);
             return fail(ARTEA_GPU_ECUDA, "row norms failed");
         }
-        ix->bf = bf_cache_create(ix->d_xsq, num_vectors, std::max(sms, 1));
+        ix->bf = bf_cache_create(device, ix->d_xsq, num_vectors, std::max(sms, 1));
     }
-    if (!ix->bf) ix->bf = bf_cache_create(nullptr, 0, 1);
+    if (!ix->bf) ix->bf = bf_cache_create(device, nullptr, 0, 1);
     *out = ix;
     return ARTEA_GPU_OK;
 }

@@ -30,8 +30,9 @@ namespace {
 constexpr int kBfQueries = 8;        // queries per CTA
 constexpr int kBfThreads = 128;      // rows per round (one per thread)
 constexpr uint32_t kBfMaxTopk = 1024;
-constexpr uint32_t kFilterRows = 8192;   // fewer rows: the scan
-constexpr uint32_t kFilterQueries = 16;  // fewer queries: the scan, unless the index's rows are rounded already
+constexpr uint32_t kFilterRows = 8192;   // fewer rows: no filter
+constexpr uint32_t kFewRows = 1024;      // fewer rows: the scan
+constexpr uint32_t kFilterQueries = 4;   // fewer queries: bf_few, unless the index's rows are rounded already
 constexpr uint64_t kMaxKey = ~0ull;
 // CandidateEntry() (router/data_structures/candidate_entry.hpp:72-74): vid =
 // invalid_vertex_id (all ones), distance 0 -- the padding of batch rows whose
@@ -284,12 +285,13 @@ __global__ void __launch_bounds__(256) bf_merge_kernel(const uint64_t* __restric
     extern __shared__ __align__(16) unsigned char bf_smem[];
     uint64_t* keys = reinterpret_cast<uint64_t*>(bf_smem);   // pow2 >= segments * k
     const uint32_t q = blockIdx.x;
-    for (uint32_t i = threadIdx.x; i < pow2; i += blockDim.x) keys[i] = kMaxKey;
-    __syncthreads();
-    for (uint32_t s = 0; s < segments; ++s) {
-        const uint32_t n = part_n[static_cast<size_t>(q) * segments + s];
-        const uint64_t* src = part + (static_cast<size_t>(q) * segments + s) * k;
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) keys[s * k + i] = src[i];
+    // (Every key on its own: walking the segments one by one waited for each one's
+    // count, 82 us at 390 segments.)
+    const uint64_t* src = part + static_cast<size_t>(q) * segments * k;
+    for (uint32_t i = threadIdx.x; i < pow2; i += blockDim.x) {
+        const uint32_t s = i / k;
+        const bool in = s < segments && i - s * k < part_n[static_cast<size_t>(q) * segments + s];
+        keys[i] = in ? src[i] : kMaxKey;
     }
     __syncthreads();
     for (uint32_t k2 = 2; k2 <= pow2; k2 <<= 1) {
@@ -329,8 +331,7 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
          const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int dev_sms, cudaStream_t st) {
     ScanFn fn = scan_kernel(metric);
     const uint32_t list_cap = next_pow2(topk + 2 * kBfThreads);
-    const size_t smem = static_cast<size_t>(kBfQueries) * list_cap * sizeof(uint64_t) +
-                        static_cast<size_t>(kBfQueries) * ix->dim * sizeof(float);
+    const size_t smem = static_cast<size_t>(kBfQueries) * (list_cap * sizeof(uint64_t) + ix->dim * sizeof(float));
     if (smem > 227u * 1024u) return fail(ARTEA_GPU_EINVAL, "brute-force tile exceeds shared memory (topk or dim too large)");
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
@@ -338,11 +339,15 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn), kBfThreads,
                                                            smem));
     const uint32_t tiles = (nq + kBfQueries - 1) / kBfQueries;
-    // Split the rows into segments until the grid covers the GPU twice over,
-    // keeping each segment >= 4096 rows and the merge within shared memory.
+    // Split the rows into segments until the grid covers the GPU twice over. A
+    // segment has at least 512 rows (4 rounds of its CTA) and 32 per result, since
+    // each hands k keys to the merge, which sorts them in shared memory: up to 4,096
+    // keys, or two segments an SM where k is large. (4,096 rows a segment left one
+    // query over 200k rows on 48 CTAs.)
     const uint32_t want = 2u * static_cast<uint32_t>(std::max(per_sm, 1) * dev_sms);
     uint32_t segments = std::max(1u, (want + tiles - 1) / tiles);
-    segments = std::min(segments, std::max(1u, n_rows / 4096u));
+    segments = std::min(segments, std::max(1u, n_rows / std::min(4096u, std::max(512u, 32u * topk))));
+    segments = std::min(segments, std::max(4096u / topk, 2u * static_cast<uint32_t>(dev_sms)));
     segments = std::min(segments, std::max(1u, 16384u / topk));
     const uint32_t seg_len = (n_rows + segments - 1) / segments;
     segments = (n_rows + seg_len - 1) / seg_len;
@@ -407,14 +412,18 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
     CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ix->device));
     const uint32_t* subset = use_subset ? d_subset : nullptr;
     // The tensor-core filter reads every row twice in FP16 and pays a rounding pass
-    // over the rows (once an index, or on every call for a subset); the scan reads
-    // them once in FP32 for every 8 queries. With fewer rows the launches decide.
-    const bool filter = n_rows >= kFilterRows && 8ull * topk <= n_rows &&
-                        (nq >= kFilterQueries || (!use_subset && bf_rows_ready(ix)));
-    if (filter) {
+    // over the rows (once an index, or on every call for a subset); bf_few reads them
+    // once in FP32 for every query; the scan once for every 8 queries, but with a
+    // sorted list a CTA. (8 queries over 1M x 128, k 100: scan 1.7 ms; filter 0.16 ms,
+    // 1.6 with the rounding.) With fewer rows the launches decide.
+    const bool many = n_rows >= kFilterRows;
+    const bool filter = many && (nq >= kFilterQueries || (!use_subset && bf_rows_ready(ix)));
+    const bool few = nq < kFilterQueries && n_rows >= kFewRows;
+    if ((filter || few) && 8ull * topk <= n_rows) {
         bool used = false;
         std::vector<uint32_t> redo;
-        if (int rc = bf_tensor(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &used, &redo))
+        if (int rc = filter ? bf_tensor(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &used, &redo)
+                            : bf_few(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &used, &redo))
             return rc;
         if (used && redo.size() <= 64) {
             for (const uint32_t q : redo)
@@ -428,21 +437,45 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
 }
 
 // Centroid of the bucket's rows (hierarchical_graph_compactor.hpp:261-300):
-// block b sums rows [b * rows_per_block, ...) of every dimension in double,
-// in row order; the final pass adds the blocks' sums in block order.
-__global__ void centroid_partial_kernel(const float* __restrict__ vecs, uint32_t dim,
-                                        const uint32_t* __restrict__ bucket, uint32_t n, uint32_t rows_per_block,
-                                        double* __restrict__ partial) {
+// block (x, y) sums rows [x * rows_per_block, ...) of dimensions [32 y, 32 y + 32) in
+// double, in row order; the final pass adds the blocks' sums in block order. One
+// warp a block and one chain of additions a lane: the order is part of the result,
+// so what is left is to keep 64 rows in flight behind it.
+constexpr int kCentroidRows = 64;
+
+__global__ void __launch_bounds__(32) centroid_partial_kernel(const float* __restrict__ vecs, uint32_t dim,
+                                                              const uint32_t* __restrict__ bucket, uint32_t n,
+                                                              uint32_t rows_per_block, double* __restrict__ partial) {
     const uint32_t r0 = blockIdx.x * rows_per_block;
     const uint32_t r1 = min(n, r0 + rows_per_block);
-    for (uint32_t d = threadIdx.x; d < dim; d += blockDim.x) {
-        double s = 0.0;
-        for (uint32_t r = r0; r < r1; ++r) {
-            const uint32_t vid = bucket ? bucket[r] : r;
-            s += static_cast<double>(vecs[static_cast<size_t>(vid) * dim + d]);
-        }
-        partial[static_cast<size_t>(blockIdx.x) * dim + d] = s;
+    const uint32_t d = blockIdx.y * 32u + threadIdx.x;
+    if (d >= dim) return;
+    double s = 0.0;
+    float next[kCentroidRows];
+#pragma unroll
+    for (int i = 0; i < kCentroidRows; ++i) {
+        const uint32_t r = min(r0 + i, r1 - 1u);
+        next[i] = __ldg(vecs + static_cast<size_t>(bucket ? bucket[r] : r) * dim + d);
     }
+    for (uint32_t base = r0; base < r1; base += kCentroidRows) {
+        float x[kCentroidRows];
+#pragma unroll
+        for (int i = 0; i < kCentroidRows; ++i) x[i] = next[i];
+#pragma unroll
+        for (int i = 0; i < kCentroidRows; ++i) {
+            const uint32_t r = min(base + kCentroidRows + i, r1 - 1u);
+            next[i] = __ldg(vecs + static_cast<size_t>(bucket ? bucket[r] : r) * dim + d);
+        }
+        if (base + kCentroidRows <= r1) {
+#pragma unroll
+            for (int i = 0; i < kCentroidRows; ++i) s += static_cast<double>(x[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kCentroidRows; ++i)
+                if (base + i < r1) s += static_cast<double>(x[i]);
+        }
+    }
+    partial[static_cast<size_t>(blockIdx.x) * dim + d] = s;
 }
 
 __global__ void centroid_final_kernel(const double* __restrict__ partial, uint32_t blocks, uint32_t dim, uint32_t n,
@@ -450,6 +483,7 @@ __global__ void centroid_final_kernel(const double* __restrict__ partial, uint32
     const double inv_n = 1.0 / static_cast<double>(n);
     for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < dim; d += gridDim.x * blockDim.x) {
         double s = 0.0;
+#pragma unroll 16
         for (uint32_t b = 0; b < blocks; ++b) s += partial[static_cast<size_t>(b) * dim + d];
         centroid[d] = static_cast<float>(s * inv_n);
     }
@@ -520,36 +554,29 @@ int artea_gpu_centroid_entry(const artea_gpu_index* index, int metric, const uin
     DeviceGuard guard(index->device);
     const uint32_t per_block = 4096;
     const uint32_t blocks = (rows + per_block - 1) / per_block;
-    uint32_t* d_bucket = nullptr;
-    double* d_partial = nullptr;
-    float* d_centroid = nullptr;
-    uint64_t* d_word = nullptr;
-    int rc = dev_alloc(&d_partial, static_cast<size_t>(blocks) * index->dim);
-    if (!rc) rc = dev_alloc(&d_centroid, index->dim);
-    if (!rc) rc = dev_alloc(&d_word, 1);
-    if (!rc && bucket) {
-        rc = dev_alloc(&d_bucket, n);
-        if (!rc && cudaMemcpy(d_bucket, bucket, sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = fail(ARTEA_GPU_ECUDA, "bucket upload failed");
-    }
-    if (!rc) {
-        centroid_partial_kernel<<<blocks, 256>>>(index->d_vecs, index->dim, d_bucket, rows, per_block, d_partial);
-        centroid_final_kernel<<<(index->dim + 255) / 256, 256>>>(d_partial, blocks, index->dim, rows, d_centroid);
-        if (cudaGetLastError() != cudaSuccess) rc = fail(ARTEA_GPU_ECUDA, "centroid kernels failed to launch");
-    }
-    if (!rc) {
-        BfWork work(index);
-        rc = bruteforce_impl(index, metric, d_centroid, 1, 1, bucket != nullptr, d_bucket, rows, d_word, work, nullptr);
-    }
+    BfWork work(index);
+    const size_t partial_bytes = sizeof(double) * static_cast<size_t>(blocks) * index->dim;
+    const size_t centroid_bytes = (sizeof(float) * index->dim + 15) / 16 * 16;
+    unsigned char* p = nullptr;
+    if (int rc = work.get(0, partial_bytes + centroid_bytes + 16 + (bucket ? sizeof(uint32_t) * n : 0), &p)) return rc;
+    double* d_partial = reinterpret_cast<double*>(p);
+    float* d_centroid = reinterpret_cast<float*>(p + partial_bytes);
+    uint64_t* d_word = reinterpret_cast<uint64_t*>(p + partial_bytes + centroid_bytes);
+    uint32_t* d_bucket = bucket ? reinterpret_cast<uint32_t*>(p + partial_bytes + centroid_bytes + 16) : nullptr;
+    if (bucket && cudaMemcpy(d_bucket, bucket, sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(ARTEA_GPU_ECUDA, "bucket upload failed");
+    centroid_partial_kernel<<<dim3(blocks, (index->dim + 31) / 32), 32>>>(index->d_vecs, index->dim, d_bucket, rows,
+                                                                         per_block, d_partial);
+    centroid_final_kernel<<<(index->dim + 31) / 32, 32>>>(d_partial, blocks, index->dim, rows, d_centroid);
+    if (cudaGetLastError() != cudaSuccess) return fail(ARTEA_GPU_ECUDA, "centroid kernels failed to launch");
+    if (int rc = bruteforce_impl(index, metric, d_centroid, 1, 1, bucket != nullptr, d_bucket, rows, d_word, work,
+                                 nullptr))
+        return rc;
     uint64_t word = 0;
-    if (!rc && cudaMemcpy(&word, d_word, sizeof(word), cudaMemcpyDeviceToHost) != cudaSuccess)
-        rc = fail(ARTEA_GPU_ECUDA, "result download failed");
-    if (!rc) *out_vid = static_cast<uint32_t>(word);
-    dev_free(d_bucket);
-    dev_free(d_partial);
-    dev_free(d_centroid);
-    dev_free(d_word);
-    return rc;
+    if (cudaMemcpy(&word, d_word, sizeof(word), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return fail(ARTEA_GPU_ECUDA, "result download failed");
+    *out_vid = static_cast<uint32_t>(word);
+    return ARTEA_GPU_OK;
 }
 
 }  // extern "C"

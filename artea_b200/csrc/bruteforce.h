@@ -12,12 +12,13 @@ struct artea_gpu_index;
 namespace artea_gpu {
 
 struct BfCache;
-BfCache* bf_cache_create(const float* d_xsq, uint32_t n, int sms);   // x.x of every row
+struct BfPool;
+BfCache* bf_cache_create(int device, const float* d_xsq, uint32_t n, int sms);   // d_xsq: x.x of every row
 void bf_cache_destroy(BfCache* c);
 
-// A call's device workspace: the index's, unless another thread's call holds it.
+// A call's device workspace: the device's, unless another thread's call holds it.
 // Slot 0: the host entry points' copies; slot 1: everything else.
-constexpr size_t kBfKeepBytes = 256u << 20;   // the index keeps no larger one
+constexpr size_t kBfKeepBytes = 256u << 20;   // no larger one is kept (per slot)
 struct BfWork {
     explicit BfWork(const artea_gpu_index* ix);
     ~BfWork();
@@ -26,7 +27,7 @@ struct BfWork {
     // At least bytes, valid until the slot's next get() or the end.
     int get(int slot, size_t bytes, unsigned char** p);
 
-    BfCache* cache;
+    BfPool* pool;
     bool held = false;
     unsigned char* own[2] = {};
 };
@@ -40,5 +41,10 @@ bool bf_rows_ready(const artea_gpu_index* ix);
 int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
               const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int sms, cudaStream_t st,
               bool* used, std::vector<uint32_t>* redo);
+
+// The same for a few queries, in FP32 throughout.
+int bf_few(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
+           const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int sms, cudaStream_t st,
+           bool* used, std::vector<uint32_t>* redo);
 
 }  // namespace artea_gpu

@@ -301,12 +301,12 @@ int artea_gpu_router_set_early_stop(artea_gpu_router* router, const float* level
  * SIMD functor. The index may have an empty graph (only its vectors are read).
  * topk in [1, 1024]. subset NULL = all vectors; a non-NULL subset with
  * n_subset 0 gives padding only. The host variant checks subset ids against
- * the vector count (EINVAL) and waits for the result. Calls with 16 queries or
+ * the vector count (EINVAL) and waits for the result. Calls with 4 queries or
  * more over 8,192 rows or more filter the rows through the tensor cores first
  * (same words); the first such call over all vectors makes an FP16 copy of them,
  * which the index keeps (2 bytes x vectors x dim rounded up to 64; without the
- * memory for it the FP32 scan serves), and an index keeps one workspace of at
- * most 512 MB for these calls. */
+ * memory for it the FP32 scan serves), and brute-force calls keep a workspace
+ * of at most 512 MB a device while an index on it exists. */
 int artea_gpu_bruteforce(const artea_gpu_index* index, int metric, const float* queries, uint32_t nq, uint32_t topk,
                          const uint32_t* subset, uint32_t n_subset, uint64_t* out);
 

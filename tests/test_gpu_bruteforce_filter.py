@@ -30,6 +30,8 @@ def _words(base, queries, k, metric, subset=None):
 def _check(base, queries, k, metric, subset=None):
     idx = DeviceIndex(vectors_only_graph(), base)
     want = _words(base, queries, k, metric, subset)
+    # Few queries while the index holds no rounded rows: FP32 throughout.
+    np.testing.assert_array_equal(idx.bruteforce(queries[:2], k, metric, subset), want[:2])
     np.testing.assert_array_equal(idx.bruteforce(queries, k, metric, subset), want)
     # Few queries, on the rounded rows that the index holds by now.
     np.testing.assert_array_equal(idx.bruteforce(queries[:3], k, metric, subset), want[:3])
@@ -70,9 +72,9 @@ def test_norms_outside_the_bounds(what, metric):
         q[9, 0] = -np.inf if what == "inf" else np.nan
     idx = DeviceIndex(vectors_only_graph(), base)
     got = idx.bruteforce(q, 20, metric)
-    # Reference: the scan (few queries on an index without rounded rows).
+    # Reference: FP32 throughout (few queries on an index without rounded rows).
     other = DeviceIndex(vectors_only_graph(), base)
-    want = np.concatenate([other.bruteforce(q[i:i + 8], 20, metric) for i in range(0, 20, 8)])
+    want = np.concatenate([other.bruteforce(q[i:i + 2], 20, metric) for i in range(0, 20, 2)])
     np.testing.assert_array_equal(got, want)
     idx.close()
     other.close()
