@@ -22,6 +22,7 @@
 
 #include <cstdint>
 #include <cfloat>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "../../include/artea_gpu.h"
@@ -418,8 +419,11 @@ __device__ __forceinline__ float finish_distance(float res, float qsq, float xsq
     return res;
 }
 
-// A row warp's registers for rows loaded ahead of their arithmetic.
+// A row warp's registers for rows loaded ahead of their arithmetic: pairs, or
+// single elements for wide rows (packing those into pairs would wait for every
+// load in turn).
 typedef f32x2 RowRegs[16];
+typedef float WideRegs[32];
 
 // Rows cvid[p, min(p + 8, cnt)) of at most kBlock chunks (kN: their number, or 0
 // for nchunks), 4 lanes a row as in batch_distances; cnt > p.
@@ -460,31 +464,26 @@ __device__ __forceinline__ void row8_distance(const DeviceGraph& g, const float*
 
 // Rows of more than kBlock chunks: 16 lanes a row, lane j owning the reference's
 // AVX-512 lane j (element 16c + j of every chunk c), so a lane keeps 32 chunks in
-// flight, one register each (chunk k of a block in half k & 1 of x[k / 2]); two
-// rows a pass. The fold's xor steps (8, 4, 2, 1) are fold16's tree (FAST: 1, 2,
+// flight; two rows a pass. The fold's xor steps (8, 4, 2, 1) are fold16's tree (FAST: 1, 2,
 // 4, 8, fold16<false>'s order), so distances are bit-identical.
 constexpr uint32_t kWideBlock = 32;
 
 // Block cb (in chunks) of rows cvid[p, min(p + 2, cnt)); cnt > p.
-__device__ __forceinline__ void wide_load(const DeviceGraph& g, const uint32_t* cvid, uint32_t p, uint32_t cnt,
-                                          uint32_t cb, RowRegs& x) {
+__device__ __forceinline__ void slice_load(const DeviceGraph& g, const uint32_t* cvid, uint32_t p, uint32_t cnt,
+                                           WideRegs& x, uint32_t cb = 0) {
     const uint32_t lane = static_cast<uint32_t>(lane_id());
     const uint32_t left = (g.dim >> 4) - cb;
     const uint32_t vid = cvid[min(p + (lane >> 4), cnt - 1u)];
     const float* row = g.vecs + static_cast<size_t>(vid) * g.dim + (lane & 15u) + 16u * cb;
 #pragma unroll
-    for (int k = 0; k < static_cast<int>(kWideBlock); k += 2) {
-        float f0 = 0.0f, f1 = 0.0f;
-        if (static_cast<uint32_t>(k) < left) f0 = __ldg(row + 16 * k);
-        if (static_cast<uint32_t>(k) + 1u < left) f1 = __ldg(row + 16 * k + 16);
-        x[k / 2] = static_cast<f32x2>(__float_as_uint(f0)) | (static_cast<f32x2>(__float_as_uint(f1)) << 32);
-    }
+    for (int k = 0; k < static_cast<int>(kWideBlock); ++k)
+        if (static_cast<uint32_t>(k) < left) x[k] = __ldg(row + 16 * k);
 }
 
 template <int kMetric, bool kExact>
-__device__ __forceinline__ void wide_distance(const DeviceGraph& g, const float* __restrict__ q, float qsq,
-                                              const uint32_t* cvid, float* cdist, uint32_t p, uint32_t cnt,
-                                              RowRegs& x) {
+__device__ __forceinline__ void slice_distance(const DeviceGraph& g, const float* __restrict__ q, float qsq,
+                                              const uint32_t* cvid, float* cdist, const uint32_t* slots, uint32_t p,
+                                              uint32_t cnt, WideRegs& x) {
     const uint32_t lane = static_cast<uint32_t>(lane_id());
     const uint32_t j = lane & 15u;
     const uint32_t nchunks = g.dim >> 4;
@@ -493,11 +492,11 @@ __device__ __forceinline__ void wide_distance(const DeviceGraph& g, const float*
     float acc = 0.0f;
     #pragma unroll 1
     for (uint32_t cb = 0; cb < nchunks; cb += kWideBlock) {
-        if (cb) wide_load(g, cvid, p, cnt, cb, x);
+        if (cb) slice_load(g, cvid, p, cnt, x, cb);
 #pragma unroll
         for (int k = 0; k < static_cast<int>(kWideBlock); ++k) {
             if (cb + k < nchunks) {
-                const float y = q[16u * (cb + k) + j], v = (k & 1) ? hi32(x[k / 2]) : lo32(x[k / 2]);
+                const float y = q[16u * (cb + k) + j], v = x[k];
                 if (kMetric == ARTEA_GPU_EUCLIDEAN_SQR || kMetric == ARTEA_GPU_EUCLIDEAN) {
                     const float d = __fsub_rn(y, v);
                     acc = __fmaf_rn(d, d, acc);
@@ -515,7 +514,7 @@ __device__ __forceinline__ void wide_distance(const DeviceGraph& g, const float*
         for (int off = 1; off < 16; off <<= 1) acc = __fadd_rn(acc, __shfl_xor_sync(kFull, acc, off));
     }
     const float res = finish_distance<kMetric, kExact>(acc, qsq, xsq);
-    if (idx < cnt && j == 0u) cdist[idx] = res;
+    if (idx < cnt && j == 0u) cdist[slots[idx]] = res;
 }
 
 // A row warp's rows of one pass, by width (128 and 96, the benchmark's, have
@@ -525,8 +524,7 @@ __device__ __forceinline__ void slice_load(const DeviceGraph& g, const uint32_t*
     const uint32_t nchunks = g.dim >> 4;
     if (nchunks == 8u) row8_load<8>(g, cvid, p, cnt, nchunks, x);
     else if (nchunks == 6u) row8_load<6>(g, cvid, p, cnt, nchunks, x);
-    else if (nchunks <= kBlock) row8_load<0>(g, cvid, p, cnt, nchunks, x);
-    else wide_load(g, cvid, p, cnt, 0, x);
+    else row8_load<0>(g, cvid, p, cnt, nchunks, x);
 }
 
 template <int kMetric, bool kExact>
@@ -536,8 +534,7 @@ __device__ __forceinline__ void slice_distance(const DeviceGraph& g, const float
     const uint32_t nchunks = g.dim >> 4;
     if (nchunks == 8u) row8_distance<kMetric, kExact, 8>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
     else if (nchunks == 6u) row8_distance<kMetric, kExact, 6>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
-    else if (nchunks <= kBlock) row8_distance<kMetric, kExact, 0>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
-    else wide_distance<kMetric, kExact>(g, q, qsq, cvid, cdist, p, cnt, x);
+    else row8_distance<kMetric, kExact, 0>(g, q, qsq, cvid, cdist, p, cnt, nchunks, x);
 }
 
 // ---------------------------------------------------------------------------
@@ -564,7 +561,11 @@ struct CoopCtl {
     uint32_t evals;     // level 0: distance evaluations
     uint32_t row_ids;   // level 0: ids in the rows expanded
     uint32_t pad[4];
-    uint32_t spec[kPadRow];   // level 0: unvisited ids of the expected row, one slice per row warp
+    // Level 0, one part of each per row warp: the unvisited ids of the expected row;
+    // the new ids of the row expanded and their slots.
+    uint32_t spec[kPadRow];
+    uint32_t ids[kPadRow];
+    uint32_t slots[kPadRow];
 };
 constexpr uint32_t kCoopWords = sizeof(CoopCtl) / 4;
 static_assert(sizeof(CoopCtl) % 16 == 0, "the control block keeps the regions after it aligned");
@@ -1644,11 +1645,14 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
 // Between B and A the row warps expand it (visited test, row loads, distances)
 // while the leader merges the previous row's accepted candidates.
 //
-// A row of 64 slots is cut into kG slices, one per row warp; a warp tests its
-// slice's ids, compacts the new ones to the front of its slice of cvid (slice
-// by slice this is row order) and writes their distances, +inf in the rest of
-// the slice (never accepted). Ids of a row are distinct, so the order in which
-// warps mark them cannot change which are new.
+// A row's 64 slots are divided over the row warps, contiguous slices for rows of at
+// most kBlock chunks (8 rows a pass, and a slice's ids in one or two sectors); in
+// turn for wide ones (2 rows a pass; near neighbours come first in a row and are
+// mostly visited, so contiguous slices would leave the last warps most of the new
+// ids: 1,000 queries of 200k x 960 25.3 against 18.2 ms). A warp tests its ids and
+// writes the new ones and their distances at their slots (or at the front of its
+// slice), which keeps row order, and +inf at the others (never accepted). Ids of a row are distinct, so the order in
+// which warps mark them cannot change which are new.
 //
 // A search by one warp is one dependent chain of about 7,000 cycles an
 // expansion on an idle GPU (row ids, visited set, two or three passes of eight
@@ -1663,7 +1667,7 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
 // -> 1.16 ms, 1,000 of 100k x 128 at queue 200 1.60 -> 1.09 ms; 10,000 queries are
 // faster with a warp each, which the autotuner finds.
 // ---------------------------------------------------------------------------
-template <int kMetric, bool kExact, int kG>
+template <int kMetric, bool kExact, int kG, bool kWide>
 __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem& sm, Visited& vs, int gw, float qsq) {
     constexpr uint32_t kSlice = kPadRow / kG;
     static_assert(kSlice <= 32, "one id per lane");
@@ -1671,17 +1675,18 @@ __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem
     const uint32_t lane = static_cast<uint32_t>(lane_id());
     const uint32_t lt = (1u << lane) - 1u;
     CoopCtl* ctl = sm.coop;
-    uint32_t* cv = sm.cvid + gw * kSlice;
-    float* cd = sm.cdist + gw * kSlice;
+    uint32_t* ids = (kWide ? ctl->ids : sm.cvid) + gw * kSlice;
+    uint32_t* slots = ctl->slots + gw * kSlice;
     uint32_t* spec = ctl->spec + gw * kSlice;
-    const uint32_t* slice = g.l0pad + gw * kSlice + lane;
+    const uint32_t slot = kWide ? lane * kG + gw : gw * kSlice + lane;   // of this lane's id
+    const uint32_t* slice = g.l0pad + slot;
     const bool has = lane < kSlice;
-    const uint32_t pass = (g.dim >> 4) > kBlock ? 2u : 8u;   // rows a pass
+    constexpr uint32_t pass = kWide ? 2u : 8u;   // rows a pass
     uint32_t pf_vid = kVidMask, pf_id = 0xffffffffu, spec_mask = 0u;
     uint32_t evals = 0, row_ids = 0;
-    RowRegs x;
+    std::conditional_t<kWide, WideRegs, RowRegs> x;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = 0ull;
+    for (int k = 0; k < (kWide ? 32 : 16); ++k) x[k] = 0;
     for (;;) {
         team_wait(kNextBarrier, kG + 1);   // B
         const uint32_t next = ctl->next;
@@ -1695,16 +1700,27 @@ __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem
         const bool is_new = team_test_and_set(vs, &ctl->list_n, id, id < g.n);
         const uint32_t b = __ballot_sync(kFull, is_new);
         const uint32_t cnt = __popc(b);
-        if (is_new) cv[__popc(b & lt)] = id;
-        if (has && lane >= cnt) cd[lane] = INFINITY;
+        if (kWide) {
+            if (has) sm.cdist[slot] = INFINITY;
+            if (is_new) {
+                const uint32_t k = __popc(b & lt);
+                ids[k] = id;
+                slots[k] = slot;
+                sm.cvid[slot] = id;
+            }
+        } else {   // compacted to the front of the slice: row order still
+            if (is_new) ids[__popc(b & lt)] = id;
+            if (has && lane >= cnt) sm.cdist[slot] = INFINITY;
+        }
         __syncwarp();
         // The rows loaded ahead are the expansion's when the guess was right
         // and no id was marked in between.
-        if (cnt && !(hit && b == spec_mask)) slice_load(g, cv, 0, cnt, x);
+        if (cnt && !(hit && b == spec_mask)) slice_load(g, ids, 0, cnt, x);
         #pragma unroll 1
         for (uint32_t p = 0; p < cnt; p += pass) {
-            if (p) slice_load(g, cv, p, cnt, x);
-            slice_distance<kMetric, kExact>(g, sm.q, qsq, cv, cd, p, cnt, x);
+            if (p) slice_load(g, ids, p, cnt, x);
+            if constexpr (kWide) slice_distance<kMetric, kExact>(g, sm.q, qsq, ids, sm.cdist, slots, p, cnt, x);
+            else slice_distance<kMetric, kExact>(g, sm.q, qsq, ids, sm.cdist + gw * kSlice, p, cnt, x);
         }
         __syncwarp();
         team_arrive(kRowsBarrier, kG + 1);   // A
@@ -1718,6 +1734,14 @@ __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem
             if ((spec_mask >> lane) & 1u) spec[__popc(spec_mask & lt)] = pf_id;
             __syncwarp();
             slice_load(g, spec, 0, __popc(spec_mask), x);
+            if (kWide) {   // and all of them into L2
+                const uint32_t sn = __popc(spec_mask), lines = g.dim >> 5;   // 128-byte lines of a row
+                #pragma unroll 1
+                for (uint32_t r = 0; r < sn; ++r) {
+                    const float* row = g.vecs + static_cast<size_t>(spec[r]) * g.dim;
+                    for (uint32_t i = lane; i < lines; i += 32) prefetch_l2(row + 32u * i);
+                }
+            }
         }
     }
     if (lane == 0) {
@@ -1954,7 +1978,8 @@ __device__ void team_rows(const SearchArgs& a, const WarpSmem& sm, int warp) {
         const float qsq = ctl->qsq;
         if (cmd == kCmdQuit) break;
         if (kPad && cmd == kCmdLevel0) {
-            l0_team_rows<kMetric, kExact, kG>(a, sm, vs, warp - 1, qsq);
+            if ((a.g.dim >> 4) <= kBlock) l0_team_rows<kMetric, kExact, kG, false>(a, sm, vs, warp - 1, qsq);
+            else l0_team_rows<kMetric, kExact, kG, true>(a, sm, vs, warp - 1, qsq);
             continue;
         }
         batch_distances<kMetric, kExact, false, false, true>(a.g, sm.q, qsq, ctl->cvid, ctl->cdist, ctl->cnt, st,
