@@ -273,136 +273,10 @@ struct Stage {
     uint32_t phase;      // parity of the next phase to wait for
 };
 
-// Loads of the next expansion's rows, issued ahead of its distance phase so
-// they are in flight while the warp merges the current batch. With kRegs, the
-// first pass's first block of chunks (rows cvid[0, 8), one float4 per chunk
-// and lane) is loaded into x, which batch_distances then consumes (kPre);
-// without, those rows' first 512 bytes are prefetched into L2 (one 128-byte
-// line per lane). With l2_next, the second pass's rows (cvid[8, 16)) are
-// prefetched into L2 as well.
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-template <bool kRegs>
-__device__ __forceinline__ void dist_preload(const DeviceGraph& g, const uint32_t* cvid, uint32_t cnt,
-                                             ulonglong2 (&x)[kBlock], bool l2_next) {
-    const int lane = lane_id();
-    const uint32_t r = static_cast<uint32_t>(lane) >> 2;
-    const uint32_t gi = lane & 3;
-    const uint32_t dim = g.dim;
-    const uint32_t off = 128u * gi;   // byte offset of this lane's line in a row
-    if (kRegs) {
-        const uint32_t nchunks = dim >> 4;
-        const bool valid = r < cnt;
-        const uint32_t vid = valid ? cvid[r] : 0u;
-        const float* row = g.vecs + static_cast<size_t>(vid) * dim + 4 * gi;
-#pragma unroll
-        for (int k = 0; k < kBlock; ++k) {
-            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(row + 16 * k);
-            x[k] = (valid && static_cast<uint32_t>(k) < nchunks) ? __ldg(src) : make_ulonglong2(0ull, 0ull);
-        }
-    } else if (r < cnt && off < dim * 4u) {
-        prefetch_l2(reinterpret_cast<const char*>(g.vecs + static_cast<size_t>(cvid[r]) * dim) + off);
-    }
-    if (l2_next && cnt > 8u) {
-        const uint32_t r2 = 8u + r;
-        if (r2 < cnt && off < dim * 4u)
-            prefetch_l2(reinterpret_cast<const char*>(g.vecs + static_cast<size_t>(cvid[r2]) * dim) + off);
-    }
-}
-
-// Distances for cnt candidates (ids in cvid, shared memory) into cdist, one
-// pass of 8 rows at a time: passes pass0, pass0 + stride, ... (the warps of a
-// cooperative search split the passes; one warp alone takes them all). With
-// kPre, the first pass's first block of chunks is taken from pre (loaded by
-// dist_preload<true> on the same cvid) instead of being loaded here.
-template <int kMetric, bool kExact, bool kStage, bool kPre = false, bool kSplit = false>
-__device__ void batch_distances(const DeviceGraph& g, const float* __restrict__ q, float qsq,
-                                const uint32_t* cvid, float* cdist, uint32_t cnt, Stage& st, int* error,
-                                const ulonglong2 (*pre)[kBlock] = nullptr, uint32_t pass0 = 0,
-                                uint32_t stride = 1) {
-    if (!kSplit) {
-        pass0 = 0;
-        stride = 1;
-    }
-    const int lane = lane_id();
-    const int r = lane >> 2;
-    const int gi = lane & 3;
-    const uint32_t dim = g.dim;
-    const uint32_t nchunks = dim >> 4;
-    const uint32_t sstride = dim + kStagePad;
-    #pragma unroll 1
-    for (uint32_t p = 8u * pass0; p < cnt; p += 8u * stride) {
-        const uint32_t idx = p + r;
-        const bool valid = idx < cnt;
-        const uint32_t vid = valid ? cvid[idx] : 0u;
-        // x.x of the row, stored at index creation in this kernel's exact
-        // summation order (row_sqnorm_kernel); loaded ahead of the row.
-        const float xsq = (kMetric == ARTEA_GPU_COSINE && valid) ? __ldg(g.xsq + vid) : 1.0f;
-        const float* row;
-        if (kStage) {
-            // The stage's previous contents have been read by every lane
-            // (generic proxy) before the async proxy overwrites them.
-            const uint32_t nrows = min(kStageRows, cnt - p);
-            __syncwarp();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            if (lane == 0) mbar_expect(st.mbar, nrows * dim * 4u);
-            __syncwarp();
-            if (static_cast<uint32_t>(lane) < nrows)
-                bulk_row_copy(smem_addr(st.buf + lane * sstride), g.vecs + static_cast<size_t>(cvid[p + lane]) * dim,
-                              dim * 4u, st.mbar);
-            if (!mbar_wait(st.mbar, st.phase)) {
-                set_error(error, kErrTimeout);
-                mbar_wait(st.mbar, st.phase);   // a second bounded wait for the copies in flight
-            }
-            st.phase ^= 1u;
-            row = st.buf + r * sstride + 4 * gi;
-        } else {
-            row = g.vecs + static_cast<size_t>(vid) * dim + 4 * gi;
-        }
-        const float* qq = q + 4 * gi;
-        f32x2 A01 = 0ull, A23 = 0ull;   // L2: diff^2; dot/cos: q*x   (+0.0f pairs)
-        #pragma unroll 1
-        for (uint32_t cb = 0; cb < nchunks; cb += kBlock) {
-            ulonglong2 x[kBlock];
-            if (kPre && p == 0 && cb == 0) {
-#pragma unroll
-                for (int k = 0; k < kBlock; ++k) x[k] = (*pre)[k];
-            } else {
-#pragma unroll
-                for (int k = 0; k < kBlock; ++k) {
-                    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(row + 16 * (cb + k));
-                    x[k] = (valid && cb + k < nchunks) ? (kStage ? *src : __ldg(src)) : make_ulonglong2(0ull, 0ull);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kBlock; ++k) {
-                if (cb + k < nchunks) {
-                    const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(qq + 16 * (cb + k));
-                    accumulate<kMetric>(x[k], y, A01, A23);
-                }
-            }
-        }
-        const float a0 = lo32(A01), a1 = hi32(A01), a2 = lo32(A23), a3 = hi32(A23);
-        float res = fold16<kExact>(a0, a1, a2, a3);
-        if (kMetric == ARTEA_GPU_EUCLIDEAN) {
-            res = __fsqrt_rn(res);
-        } else if (kMetric == ARTEA_GPU_DOT) {
-            res = -res;
-        } else if (kMetric == ARTEA_GPU_COSINE) {
-            // utils/simd_distance.hpp:263-274
-            const float denom = __fsqrt_rn(__fmul_rn(qsq, xsq));
-            res = denom > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(res, denom)) : 1.0f;
-        }
-        if (valid && gi == 0) cdist[idx] = res;
-    }
-    __syncwarp();
-}
-
 // ---------------------------------------------------------------------------
-// Distances of a row warp's few rows (team search). One warp per scheduler
-// issues an instruction every 4-6 cycles here, so what counts is instructions:
+// Distances of rows of at most kBlock chunks. A warp issues an instruction every
+// 4-8 cycles in a search (one warp a scheduler in a team, five otherwise, each one
+// dependent chain), so what counts is instructions:
 // lanes without a row of their own repeat the last one (the same addresses, no
 // extra traffic) instead of being masked, and rows are loaded apart from the
 // arithmetic, ahead of it.
@@ -460,6 +334,154 @@ __device__ __forceinline__ void row8_distance(const DeviceGraph& g, const float*
     const float res = finish_distance<kMetric, kExact>(fold16<kExact>(lo32(A01), hi32(A01), lo32(A23), hi32(A23)), qsq,
                                                        xsq);
     if (idx < cnt && (lane & 3u) == 0u) cdist[idx] = res;
+}
+
+// Loads of the next expansion's rows, issued ahead of its distance phase so
+// they are in flight while the warp merges the current batch. With kRegs, the
+// first pass's first block of chunks (rows cvid[0, 8), one float4 per chunk
+// and lane) is loaded into x, which batch_distances then consumes (kPre);
+// without, those rows' first 512 bytes are prefetched into L2 (one 128-byte
+// line per lane). With l2_next, the second pass's rows (cvid[8, 16)) are
+// prefetched into L2 as well.
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+template <bool kRegs>
+__device__ __forceinline__ void dist_preload(const DeviceGraph& g, const uint32_t* cvid, uint32_t cnt,
+                                             RowRegs& x, bool l2_next) {
+    const int lane = lane_id();
+    const uint32_t r = static_cast<uint32_t>(lane) >> 2;
+    const uint32_t gi = lane & 3;
+    const uint32_t dim = g.dim;
+    const uint32_t off = 128u * gi;   // byte offset of this lane's line in a row
+    if (kRegs) {
+        const uint32_t nchunks = dim >> 4;
+        if (cnt) {
+            if (nchunks == 8u) row8_load<8>(g, cvid, 0, cnt, nchunks, x);
+            else if (nchunks == 6u) row8_load<6>(g, cvid, 0, cnt, nchunks, x);
+            else row8_load<0>(g, cvid, 0, cnt, min(nchunks, static_cast<uint32_t>(kBlock)), x);
+        }
+    } else if (r < cnt && off < dim * 4u) {
+        prefetch_l2(reinterpret_cast<const char*>(g.vecs + static_cast<size_t>(cvid[r]) * dim) + off);
+    }
+    if (l2_next && cnt > 8u) {
+        const uint32_t r2 = 8u + r;
+        if (r2 < cnt && off < dim * 4u)
+            prefetch_l2(reinterpret_cast<const char*>(g.vecs + static_cast<size_t>(cvid[r2]) * dim) + off);
+    }
+}
+
+// Distances for cnt candidates (ids in cvid, shared memory) into cdist, one
+// pass of 8 rows at a time: passes pass0, pass0 + stride, ... (the warps of a
+// cooperative search split the passes; one warp alone takes them all). With
+// kPre, the first pass's first block of chunks is taken from pre (loaded by
+// dist_preload<true> on the same cvid) instead of being loaded here.
+// The whole batch for rows of kN chunks: about 50 instructions a pass less than the
+// masked loads below (1M x 128, 10,000 queries, 96 registers: queue 100 4.30 -> 3.55
+// ms, pipelined 3.60 -> 3.41; 1M x 96 cosine uneven batch 5.95 -> 5.55 ms).
+template <int kMetric, bool kExact, bool kPre, int kN>
+__device__ __forceinline__ void narrow_distances(const DeviceGraph& g, const float* __restrict__ q, float qsq,
+                                                 const uint32_t* cvid, float* cdist, uint32_t cnt,
+                                                 const RowRegs* pre) {
+    RowRegs x;
+    if (kPre) {
+#pragma unroll
+        for (int k = 0; k < 2 * kN; ++k) x[k] = (*pre)[k];
+    }
+    #pragma unroll 1
+    for (uint32_t p = 0; p < cnt; p += 8u) {
+        if (!kPre || p) row8_load<kN>(g, cvid, p, cnt, kN, x);
+        row8_distance<kMetric, kExact, kN>(g, q, qsq, cvid, cdist, p, cnt, kN, x);
+    }
+    __syncwarp();
+}
+
+template <int kMetric, bool kExact, bool kStage, bool kPre = false, bool kSplit = false, bool kNarrow = false>
+__device__ void batch_distances(const DeviceGraph& g, const float* __restrict__ q, float qsq,
+                                const uint32_t* cvid, float* cdist, uint32_t cnt, Stage& st, int* error,
+                                const RowRegs* pre = nullptr, uint32_t pass0 = 0,
+                                uint32_t stride = 1) {
+    if (!kSplit) {
+        pass0 = 0;
+        stride = 1;
+    }
+    const int lane = lane_id();
+    const int r = lane >> 2;
+    const int gi = lane & 3;
+    const uint32_t dim = g.dim;
+    const uint32_t nchunks = dim >> 4;
+    const uint32_t sstride = dim + kStagePad;
+    if (kNarrow && !kStage && !kSplit) {   // level 0 of the benchmark's widths: 128 and 96
+        if (nchunks == 8u) return narrow_distances<kMetric, kExact, kPre, 8>(g, q, qsq, cvid, cdist, cnt, pre);
+        if (nchunks == 6u) return narrow_distances<kMetric, kExact, kPre, 6>(g, q, qsq, cvid, cdist, cnt, pre);
+    }
+    #pragma unroll 1
+    for (uint32_t p = 8u * pass0; p < cnt; p += 8u * stride) {
+        const uint32_t idx = p + r;
+        const bool valid = idx < cnt;
+        const uint32_t vid = valid ? cvid[idx] : 0u;
+        // x.x of the row, stored at index creation in this kernel's exact
+        // summation order (row_sqnorm_kernel); loaded ahead of the row.
+        const float xsq = (kMetric == ARTEA_GPU_COSINE && valid) ? __ldg(g.xsq + vid) : 1.0f;
+        const float* row;
+        if (kStage) {
+            // The stage's previous contents have been read by every lane
+            // (generic proxy) before the async proxy overwrites them.
+            const uint32_t nrows = min(kStageRows, cnt - p);
+            __syncwarp();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (lane == 0) mbar_expect(st.mbar, nrows * dim * 4u);
+            __syncwarp();
+            if (static_cast<uint32_t>(lane) < nrows)
+                bulk_row_copy(smem_addr(st.buf + lane * sstride), g.vecs + static_cast<size_t>(cvid[p + lane]) * dim,
+                              dim * 4u, st.mbar);
+            if (!mbar_wait(st.mbar, st.phase)) {
+                set_error(error, kErrTimeout);
+                mbar_wait(st.mbar, st.phase);   // a second bounded wait for the copies in flight
+            }
+            st.phase ^= 1u;
+            row = st.buf + r * sstride + 4 * gi;
+        } else {
+            row = g.vecs + static_cast<size_t>(vid) * dim + 4 * gi;
+        }
+        const float* qq = q + 4 * gi;
+        f32x2 A01 = 0ull, A23 = 0ull;   // L2: diff^2; dot/cos: q*x   (+0.0f pairs)
+        #pragma unroll 1
+        for (uint32_t cb = 0; cb < nchunks; cb += kBlock) {
+            ulonglong2 x[kBlock];
+            if (kPre && p == 0 && cb == 0) {
+#pragma unroll
+                for (int k = 0; k < kBlock; ++k) x[k] = make_ulonglong2((*pre)[2 * k], (*pre)[2 * k + 1]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < kBlock; ++k) {
+                    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(row + 16 * (cb + k));
+                    x[k] = (valid && cb + k < nchunks) ? (kStage ? *src : __ldg(src)) : make_ulonglong2(0ull, 0ull);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kBlock; ++k) {
+                if (cb + k < nchunks) {
+                    const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(qq + 16 * (cb + k));
+                    accumulate<kMetric>(x[k], y, A01, A23);
+                }
+            }
+        }
+        const float a0 = lo32(A01), a1 = hi32(A01), a2 = lo32(A23), a3 = hi32(A23);
+        float res = fold16<kExact>(a0, a1, a2, a3);
+        if (kMetric == ARTEA_GPU_EUCLIDEAN) {
+            res = __fsqrt_rn(res);
+        } else if (kMetric == ARTEA_GPU_DOT) {
+            res = -res;
+        } else if (kMetric == ARTEA_GPU_COSINE) {
+            // utils/simd_distance.hpp:263-274
+            const float denom = __fsqrt_rn(__fmul_rn(qsq, xsq));
+            res = denom > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(res, denom)) : 1.0f;
+        }
+        if (valid && gi == 0) cdist[idx] = res;
+    }
+    __syncwarp();
 }
 
 // Rows of more than kBlock chunks: 16 lanes a row, lane j owning the reference's
@@ -1566,7 +1588,7 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
     uint32_t ids0 = __ldg(pad + static_cast<size_t>(cur) * kPadRow);
     uint32_t ids1 = __ldg(pad + static_cast<size_t>(cur) * kPadRow + 32);
     uint32_t cnt = collect_pad_row(g, vs, ids0, ids1, cv, ct, a.error);
-    ulonglong2 pre[kBlock];
+    RowRegs pre;
     dist_preload<kRegs>(g, cv, cnt, pre, l2_next);
     pc.lap(kPhCollect);
     // The predicted entry after the one being expanded: its index (-1: none),
@@ -1575,7 +1597,7 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
     uint32_t pf_vid = kVidMask, pf_ids0 = 0u, pf_ids1 = 0u;
     for (uint32_t it = 0;; ++it) {
         if (it > g.n) { set_error(a.error, kErrBound); break; }
-        if (cnt) batch_distances<kMetric, kExact, false, kRegs>(g, sm.q, qsq, cv, cd, cnt, st, a.error, &pre);
+        if (cnt) batch_distances<kMetric, kExact, false, kRegs, false, true>(g, sm.q, qsq, cv, cd, cnt, st, a.error, &pre);
         ct.dist_evals += cnt;
         pc.lap(kPhDist);
         const uint32_t m = cnt ? queue_accept(q, cv, cd, cnt, sm.bd, sm.bv) : 0u;
@@ -2199,7 +2221,11 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
                         ++trows;
                     }
                     if (cnt == 0) continue;
-                    dist_call<kMetric, kExact, kStage, kG>(g, sm.q, qsq, cvid, cdist, cnt, st, a.error, sm.coop);
+                    if constexpr (kG == 0)
+                        batch_distances<kMetric, kExact, kStage, false, false, true>(g, sm.q, qsq, cvid, cdist, cnt, st,
+                                                                                    a.error);
+                    else
+                        dist_call<kMetric, kExact, kStage, kG>(g, sm.q, qsq, cvid, cdist, cnt, st, a.error, sm.coop);
                     ct.dist_evals += cnt;
                     if (kTrace) {
                         #pragma unroll 1
