@@ -1121,8 +1121,25 @@ __device__ __forceinline__ int queue_pop_peek(Queue& q, int* next) {
 // lb yields exactly the state the sequential pushes leave (entries trimmed
 // in between are worse than every later lb).
 //
+// exact_pre: the second sum for candidate j < cnt, four candidates a step;
+// the slots past cnt that the last step reads are not before j. (A walk over
+// the earlier improving lanes by shuffles took a step per candidate.)
+//
 // queue_accept writes the accepted candidates (m <= cnt <= kCandBatch), in
 // candidate order, to bd/bv and returns m.
+__device__ __forceinline__ uint32_t exact_pre(const float* cdist, uint32_t cnt, uint32_t j, float d) {
+    uint32_t pre = 0;
+    #pragma unroll 1
+    for (uint32_t i = 0; i < cnt; i += 4) {
+        const float4 c = *reinterpret_cast<const float4*>(cdist + i);
+        pre += (i < j) & (c.x <= d) ? 1u : 0u;
+        pre += (i + 1u < j) & (c.y <= d) ? 1u : 0u;
+        pre += (i + 2u < j) & (c.z <= d) ? 1u : 0u;
+        pre += (i + 3u < j) & (c.w <= d) ? 1u : 0u;
+    }
+    return pre;
+}
+
 __device__ inline uint32_t queue_accept(const Queue& q, const uint32_t* cvid, const float* cdist, uint32_t cnt,
                                         float* bd, uint32_t* bv) {
     const int lane = lane_id();
@@ -1157,24 +1174,7 @@ __device__ inline uint32_t queue_accept(const Queue& q, const uint32_t* cvid, co
         }
         const bool undecided = improving && !acc && ub != 0;
         if (__any_sync(kFull, undecided)) {
-            // Exact pre: earlier chunks from shared memory, this chunk by
-            // shuffles over the improving lanes only.
-            uint32_t pre = 0;
-            if (improving_before) {
-                #pragma unroll 1
-                for (uint32_t i = 0; i < base; ++i) pre += cdist[i] <= d ? 1u : 0u;
-            }
-            #pragma unroll 1
-            for (uint32_t bits = imask & lt_mask; __any_sync(kFull, bits != 0);) {
-                // each lane walks its own set of earlier improving lanes; shuffles
-                // need every lane, so lanes take turns through a uniform loop.
-                const int k = bits ? __ffs(bits) - 1 : 0;
-                const float dk = __shfl_sync(kFull, d, k);
-                if (bits) {
-                    pre += dk <= d ? 1u : 0u;
-                    bits &= bits - 1;
-                }
-            }
+            const uint32_t pre = exact_pre(cdist, cnt, j, d);
             if (undecided && pre < q.L) {
                 const uint32_t idx = q.L - pre - 1;
                 acc = idx >= tn || ent_d(q.e[idx]) > d;
@@ -1395,29 +1395,6 @@ __device__ inline bool queue_push_batch(Queue& q, uint32_t* cvid, float* cdist, 
     return queue_merge(q, bd, bv, queue_accept(q, cvid, cdist, cnt, bd, bv));
 }
 
-// The smallest accepted entry of bd/bv[0, m) by (dist, vid), m >= 1: its index
-// (in every lane), distance and vid word.
-__device__ __forceinline__ uint32_t batch_argmin(const float* bd, const uint32_t* bv, uint32_t m, float* d_out,
-                                                 uint32_t* v_out) {
-    const int lane = lane_id();
-    float md = INFINITY;
-    uint32_t mv = 0xffffffffu, mi = 0xffffffffu;
-    for (uint32_t k = lane; k < m; k += 32) {
-        const float d = bd[k];
-        const uint32_t v = bv[k];
-        if (mi == 0xffffffffu || entry_less(d, v, md, mv)) { md = d; mv = v; mi = k; }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        const float od = __shfl_xor_sync(kFull, md, off);
-        const uint32_t ov = __shfl_xor_sync(kFull, mv, off);
-        const uint32_t oi = __shfl_xor_sync(kFull, mi, off);
-        if (oi != 0xffffffffu && (mi == 0xffffffffu || entry_less(od, ov, md, mv))) { md = od; mv = ov; mi = oi; }
-    }
-    *d_out = md;
-    *v_out = mv;
-    return mi;
-}
-
 // ---------------------------------------------------------------------------
 // Row lookup: fetch_level_nbrs (index/compact_structure/hierarchical_graph.hpp:99-108).
 // ---------------------------------------------------------------------------
@@ -1548,6 +1525,106 @@ __device__ __forceinline__ uint32_t collect_pad_row(const DeviceGraph& g, Visite
     return collect_row64_unique(g, vs, ids0, ids1, len, cvid, error);
 }
 
+// Order-preserving unsigned key of a distance (-0 and +0 alike).
+__device__ __forceinline__ uint32_t dist_key(float d) {
+    const uint32_t u = __float_as_uint(d + 0.0f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ bool head_less(uint32_t ka, uint32_t va, uint32_t kb, uint32_t vb) {
+    return ka < kb || (ka == kb && va < vb);
+}
+
+// queue_accept over slots [0, cnt) of cvid/cdist (two a lane), plus the smallest
+// accepted candidate by (dist, vid), and with kTwo the second smallest: their
+// distance keys and vids (~0u when absent). The candidates stay in registers:
+// the decision is on the warp's own chain between a row's distances and the
+// next row's collection, where a pass through shared memory and a shuffle tree
+// for the smallest cost ~250 cycles more than two warp reductions. Before and
+// after in the one-warp loop (fixed launches): 1M x 128, 10,000 queries, queue
+// 100: 3.41 -> 3.23 ms; queue 400: 12.40 -> 11.81 ms; 96 elements, cosine,
+// early stop: 5.56 -> 5.29 ms.
+struct Batch {
+    float d[2];
+    uint32_t v[2];
+    uint32_t acc[2];          // accepted lanes of each half
+    uint32_t m;               // accepted candidates
+    uint32_t k1, v1, k2, v2;
+};
+
+template <bool kTwo>
+__device__ __forceinline__ void register_accept(const Queue& q, const uint32_t* cvid, const float* cdist, uint32_t cnt,
+                                                Batch& s) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t tn = min(q.n, q.L);
+    const float lim = q.n >= q.L ? q.lb : INFINITY;
+    s.k1 = s.v1 = s.k2 = s.v2 = 0xffffffffu;
+    s.m = 0;
+    s.d[0] = lane < cnt ? cdist[lane] : INFINITY;
+    s.d[1] = lane + 32u < cnt ? cdist[lane + 32] : INFINITY;
+    s.v[0] = cvid[lane];
+    s.v[1] = cvid[lane + 32];
+    s.acc[0] = s.acc[1] = 0u;
+    const uint32_t imp0 = __ballot_sync(kFull, s.d[0] < lim), imp1 = __ballot_sync(kFull, s.d[1] < lim);
+    if ((imp0 | imp1) == 0u) return;   // three of four rows improve nothing
+    // See queue_accept: ub bounds pre, and only lanes it leaves undecided need
+    // the exact count.
+    bool open = false;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const bool improving = s.d[t] < lim;
+        const uint32_t ub = (t ? __popc(imp0) : 0u) + __popc((t ? imp1 : imp0) & lt_mask);
+        bool acc = false;
+        if (improving && ub < q.L) {
+            const uint32_t idx = q.L - ub - 1;
+            acc = idx >= tn || ent_d(q.e[idx]) > s.d[t];
+        }
+        open |= improving && !acc && ub != 0u;
+        s.acc[t] = __ballot_sync(kFull, acc);
+    }
+    if (__any_sync(kFull, open)) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float d = s.d[t];
+            const uint32_t pre = exact_pre(cdist, cnt, lane + 32u * t, d);
+            bool acc = false;
+            if (d < lim && pre < q.L) {
+                const uint32_t idx = q.L - pre - 1u;
+                acc = idx >= tn || ent_d(q.e[idx]) > d;
+            }
+            s.acc[t] = __ballot_sync(kFull, acc);
+        }
+    }
+    s.m = __popc(s.acc[0]) + __popc(s.acc[1]);
+    if (s.m == 0u) return;
+    uint32_t key0 = (s.acc[0] >> lane) & 1u ? dist_key(s.d[0]) : 0xffffffffu;
+    uint32_t key1 = (s.acc[1] >> lane) & 1u ? dist_key(s.d[1]) : 0xffffffffu;
+    s.k1 = __reduce_min_sync(kFull, min(key0, key1));
+    s.v1 = __reduce_min_sync(kFull, min(key0 == s.k1 ? s.v[0] : 0xffffffffu, key1 == s.k1 ? s.v[1] : 0xffffffffu));
+    if (kTwo && s.m > 1u) {
+        if (s.v[0] == s.v1) key0 = 0xffffffffu;
+        if (s.v[1] == s.v1) key1 = 0xffffffffu;
+        s.k2 = __reduce_min_sync(kFull, min(key0, key1));
+        s.v2 = __reduce_min_sync(kFull, min(key0 == s.k2 ? s.v[0] : 0xffffffffu,
+                                            key1 == s.k2 ? s.v[1] : 0xffffffffu));
+    }
+}
+
+// The accepted candidates, in slot order, to bd/bv; the one popped already
+// (`popped`) with the explored bit.
+__device__ __forceinline__ void write_accepted(const Batch& s, uint32_t popped, float* bd, uint32_t* bv) {
+    const uint32_t lane = static_cast<uint32_t>(lane_id());
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        if ((s.acc[t] >> lane) & 1u) {
+            const uint32_t k = (t ? __popc(s.acc[0]) : 0u) + __popc(s.acc[t] & lt);
+            bd[k] = s.d[t];
+            bv[k] = s.v[t] | (s.v[t] == popped ? kExplored : 0u);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Level-0 beam search, pipelined across expansions (single_layer_router.hpp:
 // 145-163, beam_loop.hpp:90-119), for graphs whose level-0 rows hold at most 64
@@ -1595,27 +1672,21 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
     // vid and ids.
     int p2 = -1;
     uint32_t pf_vid = kVidMask, pf_ids0 = 0u, pf_ids1 = 0u;
+    uint32_t p2_key = 0xffffffffu;   // its distance key (~0u: none)
     for (uint32_t it = 0;; ++it) {
         if (it > g.n) { set_error(a.error, kErrBound); break; }
         if (cnt) batch_distances<kMetric, kExact, false, kRegs, false, true>(g, sm.q, qsq, cv, cd, cnt, st, a.error, &pre);
         ct.dist_evals += cnt;
         pc.lap(kPhDist);
-        const uint32_t m = cnt ? queue_accept(q, cv, cd, cnt, sm.bd, sm.bv) : 0u;
+        Batch s;
+        register_accept<false>(q, cv, cd, cnt, s);
+        const uint32_t m = s.m;
         // The next pop: min(p2, smallest accepted), or termination.
-        bool take_new = false;
-        uint32_t next = kVidMask;
-        if (m) {
-            float bdm;
-            uint32_t bvm;
-            const uint32_t bi = batch_argmin(sm.bd, sm.bv, m, &bdm, &bvm);
-            take_new = p2 < 0 || entry_less(bdm, bvm, ent_d(q.e[p2]), q.e[p2].x);
-            if (take_new) {
-                next = bvm & kVidMask;
-                if (lane == 0) sm.bv[bi] = bvm | kExplored;
-            }
-        }
+        const bool take_new = head_less(s.k1, s.v1, p2_key, pf_vid);
+        uint32_t next = take_new ? s.v1 : kVidMask;
+        if (m) write_accepted(s, next, sm.bd, sm.bv);
         if (!take_new && p2 >= 0) {
-            next = q.e[p2].x & kVidMask;
+            next = pf_vid;
             if (lane == 0) q.e[p2].x |= kExplored;
             q.hint = static_cast<uint32_t>(p2) + 1;
         }
@@ -1645,12 +1716,15 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
         p2 = queue_find_unexplored(q, q.hint);
         if (p2 >= 0) {
             q.hint = static_cast<uint32_t>(p2);
-            pf_vid = q.e[p2].x & kVidMask;
+            const uint2 w = q.e[p2];
+            pf_vid = w.x & kVidMask;
+            p2_key = dist_key(ent_d(w));
             pf_ids0 = __ldg(pad + static_cast<size_t>(pf_vid) * kPadRow);
             pf_ids1 = __ldg(pad + static_cast<size_t>(pf_vid) * kPadRow + 32);
         } else {
             q.hint = q.n;
             pf_vid = kVidMask;
+            p2_key = 0xffffffffu;
         }
         pc.lap(kPhPop);
         cnt = ncnt;
@@ -1773,94 +1847,6 @@ __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem
     coop_barrier(kG + 1);   // end: counts are in
 }
 
-// Order-preserving unsigned key of a distance (-0 and +0 alike).
-__device__ __forceinline__ uint32_t dist_key(float d) {
-    const uint32_t u = __float_as_uint(d + 0.0f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ bool head_less(uint32_t ka, uint32_t va, uint32_t kb, uint32_t vb) {
-    return ka < kb || (ka == kb && va < vb);
-}
-
-// queue_accept over the 64 slots of cvid/cdist (two a lane), plus the two
-// smallest accepted candidates by (dist, vid): their distance keys and vids
-// (~0u when absent). The candidates stay in registers.
-struct TeamBatch {
-    float d[2];
-    uint32_t v[2];
-    uint32_t acc[2];          // accepted lanes of each half
-    uint32_t m;               // accepted candidates
-    uint32_t k1, v1, k2, v2;
-};
-
-__device__ __forceinline__ void team_accept(const Queue& q, const uint32_t* cvid, const float* cdist, TeamBatch& s) {
-    const uint32_t lane = static_cast<uint32_t>(lane_id());
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const uint32_t tn = min(q.n, q.L);
-    const float lim = q.n >= q.L ? q.lb : INFINITY;
-    s.k1 = s.v1 = s.k2 = s.v2 = 0xffffffffu;
-    s.m = 0;
-    s.d[0] = cdist[lane];
-    s.d[1] = cdist[lane + 32];
-    s.v[0] = cvid[lane];
-    s.v[1] = cvid[lane + 32];
-    s.acc[0] = s.acc[1] = 0u;
-    const uint32_t imp0 = __ballot_sync(kFull, s.d[0] < lim), imp1 = __ballot_sync(kFull, s.d[1] < lim);
-    if ((imp0 | imp1) == 0u) return;   // three of four rows improve nothing
-    // See queue_accept: ub bounds pre, and only lanes it leaves undecided need
-    // the exact count.
-    bool open = false;
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const bool improving = s.d[t] < lim;
-        const uint32_t ub = (t ? __popc(imp0) : 0u) + __popc((t ? imp1 : imp0) & lt_mask);
-        bool acc = false;
-        if (improving && ub < q.L) {
-            const uint32_t idx = q.L - ub - 1;
-            acc = idx >= tn || ent_d(q.e[idx]) > s.d[t];
-        }
-        open |= improving && !acc && ub != 0u;
-        s.acc[t] = __ballot_sync(kFull, acc);
-    }
-    if (__any_sync(kFull, open)) {
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const float d = s.d[t];
-            const uint32_t j = lane + 32u * t;
-            uint32_t pre = 0;   // #{i < j : d_i <= d_j}, over the improving candidates
-            #pragma unroll 1
-            for (uint32_t bits = imp0; bits; bits &= bits - 1u) {
-                const uint32_t i = __ffs(bits) - 1u;
-                pre += i < j && cdist[i] <= d ? 1u : 0u;
-            }
-            #pragma unroll 1
-            for (uint32_t bits = t ? imp1 : 0u; bits; bits &= bits - 1u) {
-                const uint32_t i = 32u + __ffs(bits) - 1u;
-                pre += i < j && cdist[i] <= d ? 1u : 0u;
-            }
-            bool acc = false;
-            if (d < lim && pre < q.L) {
-                const uint32_t idx = q.L - pre - 1u;
-                acc = idx >= tn || ent_d(q.e[idx]) > d;
-            }
-            s.acc[t] = __ballot_sync(kFull, acc);
-        }
-    }
-    s.m = __popc(s.acc[0]) + __popc(s.acc[1]);
-    if (s.m == 0u) return;
-    uint32_t key0 = (s.acc[0] >> lane) & 1u ? dist_key(s.d[0]) : 0xffffffffu;
-    uint32_t key1 = (s.acc[1] >> lane) & 1u ? dist_key(s.d[1]) : 0xffffffffu;
-    s.k1 = __reduce_min_sync(kFull, min(key0, key1));
-    s.v1 = __reduce_min_sync(kFull, min(key0 == s.k1 ? s.v[0] : 0xffffffffu, key1 == s.k1 ? s.v[1] : 0xffffffffu));
-    if (s.m > 1u) {
-        if (s.v[0] == s.v1) key0 = 0xffffffffu;
-        if (s.v[1] == s.v1) key1 = 0xffffffffu;
-        s.k2 = __reduce_min_sync(kFull, min(key0, key1));
-        s.v2 = __reduce_min_sync(kFull, min(key0 == s.k2 ? s.v[0] : 0xffffffffu,
-                                            key1 == s.k2 ? s.v[1] : 0xffffffffu));
-    }
-}
-
 // An unexplored entry of the queue: distance key, vid, index (-1: absent).
 struct Head {
     uint32_t k, v;
@@ -1895,7 +1881,6 @@ template <int kG>
 __device__ __forceinline__ bool l0_team_lead(const SearchArgs& a, Queue& q, Visited& vs, const WarpSmem& sm,
                                              uint32_t cur, Counters& ct, PhaseClock& pc) {
     const uint32_t lane = static_cast<uint32_t>(lane_id());
-    const uint32_t lt = (1u << lane) - 1u;
     CoopCtl* ctl = sm.coop;
     if (lane == 0) {
         q.e[0].x |= kExplored;   // pop the cursor: the queue's only entry
@@ -1929,12 +1914,12 @@ __device__ __forceinline__ bool l0_team_lead(const SearchArgs& a, Queue& q, Visi
         pc.lap(kPhDist);
         uint32_t next = kVidMask, pf = kVidMask;
         bool take_new = false;
-        TeamBatch s;
+        Batch s;
         s.m = 0;
         if (it > a.g.n) {
             set_error(a.error, kErrBound);
         } else if (!lost) {
-            team_accept(q, sm.cvid, sm.cdist, s);
+            register_accept<true>(q, sm.cvid, sm.cdist, kPadRow, s);
             // Heads: queue (h1, h2) and batch (s.1, s.2), each ascending.
             take_new = head_less(s.k1, s.v1, h1.k, h1.v);
             next = take_new ? s.v1 : h1.v;
@@ -1953,16 +1938,7 @@ __device__ __forceinline__ bool l0_team_lead(const SearchArgs& a, Queue& q, Visi
         // Off the row warps' chain: the accepted candidates, in slot order, to
         // bd/bv for the merge; the popped entry marked explored where it lies.
         m = s.m;
-        if (m) {
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                if ((s.acc[t] >> lane) & 1u) {
-                    const uint32_t k = (t ? __popc(s.acc[0]) : 0u) + __popc(s.acc[t] & lt);
-                    sm.bd[k] = s.d[t];
-                    sm.bv[k] = s.v[t] | (take_new && s.v[t] == s.v1 ? kExplored : 0u);
-                }
-            }
-        }
+        if (m) write_accepted(s, take_new ? s.v1 : kVidMask, sm.bd, sm.bv);
         if (!take_new) {
             if (lane == 0) q.e[h1.at].x |= kExplored;
             q.hint = static_cast<uint32_t>(h1.at) + 1u;
