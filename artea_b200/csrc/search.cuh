@@ -582,7 +582,8 @@ struct CoopCtl {
     uint32_t list_n;    // level 0: ids put in the visited bitset since the last clear
     uint32_t evals;     // level 0: distance evaluations
     uint32_t row_ids;   // level 0: ids in the rows expanded
-    uint32_t pad[4];
+    uint32_t lead;      // helped search: the leader's warp
+    uint32_t pad[3];
     // Level 0, one part of each per row warp: the unvisited ids of the expected row;
     // the new ids of the row expanded and their slots.
     uint32_t spec[kPadRow];
@@ -1625,6 +1626,17 @@ __device__ __forceinline__ void write_accepted(const Batch& s, uint32_t popped, 
     }
 }
 
+// The last warp of a CTA that still has a query: the CTA's flags, in the first
+// warp's phase accumulators (a launch that measures phases has no helpers).
+constexpr int kHelpers = 3;   // row warps of a helped search: a CTA of four warps
+struct HelpFlags {
+    uint32_t taken;   // row warp numbers given to warps without a query
+    uint32_t host;    // the first of those warps: its candidate buffers hold the control block
+    uint32_t idle;    // warps without a query, host known
+    uint32_t quit;    // no warp of the CTA has a query
+};
+static_assert(sizeof(HelpFlags) <= 4 * kPhaseWords && sizeof(CoopCtl) <= 16 * kCandBatch, "both fit where they lie");
+
 // ---------------------------------------------------------------------------
 // Level-0 beam search, pipelined across expansions (single_layer_router.hpp:
 // 145-163, beam_loop.hpp:90-119), for graphs whose level-0 rows hold at most 64
@@ -1647,11 +1659,22 @@ __device__ __forceinline__ void write_accepted(const Batch& s, uint32_t popped, 
 // The chosen entry is marked explored where it lies: p2 in the array, a new
 // candidate in the batch before the merge places it.
 // ---------------------------------------------------------------------------
-// Returns true when the compact queue lost a live entry (see queue_merge).
-template <int kMetric, bool kExact, bool kRegs>
+// Returns true when the compact queue lost a live entry (see queue_merge). With
+// kHelp and `help`, the loop ends early once the other warps of the CTA have no
+// queries left: hand.first is then the next vertex to expand (marked explored,
+// its row not read) and hand.m candidates in bd/bv are still to be merged.
+struct Handover {
+    uint32_t first;   // kVidMask: the search ran to its end
+    uint32_t m;
+};
+
+template <int kMetric, bool kExact, bool kRegs, bool kHelp>
 __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& q, Visited& vs, const WarpSmem& sm,
                                                     float qsq, uint32_t cur, Counters& ct, PhaseClock& pc,
-                                                    Stage& st) {
+                                                    Stage& st, bool help, Handover& hand) {
+    extern __shared__ __align__(16) float smem[];
+    hand.first = kVidMask;
+    hand.m = 0;
     const int lane = lane_id();
     const DeviceGraph& g = a.g;
     const bool l2_next = a.pf_l2 != 0;
@@ -1675,6 +1698,9 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
     uint32_t p2_key = 0xffffffffu;   // its distance key (~0u: none)
     for (uint32_t it = 0;; ++it) {
         if (it > g.n) { set_error(a.error, kErrBound); break; }
+        bool helped = false;
+        if (kHelp && help)
+            helped = __all_sync(kFull, reinterpret_cast<const volatile HelpFlags*>(smem)->idle == kHelpers);
         if (cnt) batch_distances<kMetric, kExact, false, kRegs, false, true>(g, sm.q, qsq, cv, cd, cnt, st, a.error, &pre);
         ct.dist_evals += cnt;
         pc.lap(kPhDist);
@@ -1694,6 +1720,11 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
         // CandidateEntry::is_invalid ends the loop as the reference's pop of an
         // invalid entry does (cannot occur on validated graphs).
         const bool go = (take_new || p2 >= 0) && next != kVidMask;
+        if (kHelp && helped && go) {
+            hand.first = next;
+            hand.m = m;
+            return false;
+        }
         uint32_t ncnt = 0;
         if (go) {
             const bool hit = !take_new && next == pf_vid;
@@ -1765,7 +1796,7 @@ __device__ __forceinline__ bool l0_search_pipelined(const SearchArgs& a, Queue& 
 // ---------------------------------------------------------------------------
 template <int kMetric, bool kExact, int kG, bool kWide>
 __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem& sm, Visited& vs, int gw, float qsq) {
-    constexpr uint32_t kSlice = kPadRow / kG;
+    constexpr uint32_t kSlice = (kPadRow + kG - 1) / kG;
     static_assert(kSlice <= 32, "one id per lane");
     const DeviceGraph& g = a.g;
     const uint32_t lane = static_cast<uint32_t>(lane_id());
@@ -1776,7 +1807,7 @@ __device__ __forceinline__ void l0_team_rows(const SearchArgs& a, const WarpSmem
     uint32_t* spec = ctl->spec + gw * kSlice;
     const uint32_t slot = kWide ? lane * kG + gw : gw * kSlice + lane;   // of this lane's id
     const uint32_t* slice = g.l0pad + slot;
-    const bool has = lane < kSlice;
+    const bool has = lane < kSlice && slot < kPadRow;
     constexpr uint32_t pass = kWide ? 2u : 8u;   // rows a pass
     uint32_t pf_vid = kVidMask, pf_id = 0xffffffffu, spec_mask = 0u;
     uint32_t evals = 0, row_ids = 0;
@@ -1874,32 +1905,30 @@ __device__ __forceinline__ Head queue_head(const Queue& q, uint32_t from) {
     return h;
 }
 
-// The leader's side of the level-0 loop. On entry the queue holds the cursor
-// and the cursor is visited. Returns true when the compact queue lost a live
-// entry (see queue_merge).
+// The leader's side of the level-0 loop. `first` is the vertex to expand next,
+// visited and marked explored; m accepted candidates in bd/bv are still to be
+// merged. Returns true when the compact queue lost a live entry (see queue_merge).
 template <int kG>
 __device__ __forceinline__ bool l0_team_lead(const SearchArgs& a, Queue& q, Visited& vs, const WarpSmem& sm,
-                                             uint32_t cur, Counters& ct, PhaseClock& pc) {
+                                             uint32_t first, uint32_t m, Counters& ct, PhaseClock& pc) {
     const uint32_t lane = static_cast<uint32_t>(lane_id());
     CoopCtl* ctl = sm.coop;
     if (lane == 0) {
-        q.e[0].x |= kExplored;   // pop the cursor: the queue's only entry
-        ctl->next = cur;
+        ctl->next = first;
         ctl->pf = kVidMask;
         ctl->list_n = vs.list_overflow ? vs.list_cap + 1u : vs.list_n;
         ctl->evals = 0;
         ctl->row_ids = 0;
         ctl->cmd = kCmdLevel0;
     }
-    q.hint = 1;
     coop_barrier(kG + 1);   // start: the row warps enter the loop
     team_arrive(kNextBarrier, kG + 1);   // B
-    uint32_t m = 0;
     uint32_t guess = kVidMask;
     bool lost = false;
-    Head h1, h2;   // the queue's first two unexplored entries
-    h1.k = h1.v = h2.k = h2.v = 0xffffffffu;
-    h1.at = h2.at = -1;
+    Head h1, h2;   // the queue's first two unexplored entries (a merge finds both anew)
+    h1 = queue_head(q, m ? q.n : q.hint);
+    h2.k = h2.v = 0xffffffffu;
+    h2.at = -1;
     for (uint32_t it = 0;; ++it) {
         ct.l0_rows++;
         // The previous row's merge runs while this row's distances are computed.
@@ -1942,7 +1971,7 @@ __device__ __forceinline__ bool l0_team_lead(const SearchArgs& a, Queue& q, Visi
         if (!take_new) {
             if (lane == 0) q.e[h1.at].x |= kExplored;
             q.hint = static_cast<uint32_t>(h1.at) + 1u;
-            h1 = h2;   // (a merge finds both anew)
+            h1 = h2;
             h2.k = h2.v = 0xffffffffu;
             h2.at = -1;
         }
@@ -1987,6 +2016,79 @@ __device__ void team_rows(const SearchArgs& a, const WarpSmem& sm, int warp) {
 }
 
 // ---------------------------------------------------------------------------
+// Helped search: the end of a persistent launch of CTAs of four warps. Queries
+// differ in length (1M x 128, queue 400: 400 to 1,122 expansions) and the long
+// ones are not known beforehand, so the last quarter of a launch of 10,000
+// queries had a few warps a CTA still searching, each alone at one warp's
+// latency. A warp that finds no query left stays as a row warp; when three are
+// there, the fourth goes on with its query as their leader (rows of at most
+// kBlock chunks, graphs with fixed-stride rows). The functions below are
+// not inlined: they run once or twice a warp, and the one-warp loop keeps its
+// registers. Fixed launches, without -> with: 1M x 128, queue 100, 2,368
+// queries 1.79 -> 1.46 ms, 10,000 3.31 -> 3.06 ms; queue 400, 2,368 queries 5.40
+// -> 4.73 ms, 10,000 12.45 -> 11.9 ms; 1M x 96 cosine, queues 64-512, 10,000
+// queries 5.32 -> 5.15 ms. (Two row warps, which are there earlier, gave less:
+// 3.30, 12.8 and 5.18 ms.)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ CoopCtl* help_ctl(float* smem, uint32_t words, uint32_t dim, uint32_t cap) {
+    const uint32_t host = reinterpret_cast<const volatile HelpFlags*>(smem)->host;
+    return reinterpret_cast<CoopCtl*>(carve(smem + static_cast<size_t>(host) * words, dim, cap).cvid);
+}
+
+// A row warp, until the last query of the CTA is done.
+template <int kMetric, bool kExact>
+__device__ __noinline__ void help_rows(const SearchArgs& args, int gw) {
+    extern __shared__ __align__(16) float smem[];
+    const SearchArgs a = args;
+    const uint32_t words = warp_smem_words(a.g.dim, a.cap, a.vh_bits);
+    for (;;) {
+        coop_barrier(kHelpers + 1);   // start
+        if (reinterpret_cast<const volatile HelpFlags*>(smem)->quit) return;
+        CoopCtl* ctl = help_ctl(smem, words, a.g.dim, a.cap);
+        const uint32_t lead = ctl->lead;
+        WarpSmem sm = carve(smem + static_cast<size_t>(lead) * words, a.g.dim, a.cap);
+        sm.coop = ctl;
+        Visited vs = visited_init(a, sm, blockIdx.x * (kHelpers + 1) + lead);
+        l0_team_rows<kMetric, kExact, kHelpers, false>(a, sm, vs, gw, ctl->qsq);
+    }
+}
+
+// The rest of a query at level 0, led by `warp`. The state is copied in and out,
+// so that the one-warp loop's stays in registers.
+struct HelpState {
+    Queue q;
+    Visited vs;
+    Counters ct;
+    Handover hand;
+    float qsq;
+};
+
+template <int kG>
+__device__ __noinline__ bool help_lead(const SearchArgs& args, uint32_t warp, HelpState& h) {
+    extern __shared__ __align__(16) float smem[];
+    const SearchArgs a = args;
+    const uint32_t words = warp_smem_words(a.g.dim, a.cap, a.vh_bits);
+    WarpSmem sm = carve(smem + static_cast<size_t>(warp) * words, a.g.dim, a.cap);
+    sm.coop = help_ctl(smem, words, a.g.dim, a.cap);
+    if (lane_id() == 0) {
+        sm.coop->lead = warp;
+        sm.coop->qsq = h.qsq;
+    }
+    Queue q = h.q;
+    q.e = sm.qe;
+    Visited vs = h.vs;
+    vs.tab = reinterpret_cast<uint2*>(sm.vh);
+    Counters ct = h.ct;
+    PhaseClock pc;
+    pc.start(false, nullptr);
+    const bool lost = l0_team_lead<kG>(a, q, vs, sm, h.hand.first, h.hand.m, ct, pc);
+    h.q = q;
+    h.vs = vs;
+    h.ct = ct;
+    return lost;
+}
+
+// ---------------------------------------------------------------------------
 // One query (hierarchical_graph_router.hpp:195-248; query_l0_only :258-286).
 // ---------------------------------------------------------------------------
 // stage_phase: with kStage, the parity of the next phase of the warp's staging
@@ -1997,11 +2099,12 @@ __device__ void team_rows(const SearchArgs& a, const WarpSmem& sm, int warp) {
 // pipelined loop holds the next expansion's first pass in registers (the
 // 128-register budget) instead of prefetching it into L2. kG: row warps of a team
 // whose leader runs this (0: one warp searches alone).
-// kTrace: record the search in a.tr (the probes' trace kernel).
+// kTrace: record the search in a.tr (the probes' trace kernel). kHelp: the
+// pipelined loop may end as a helped search (`help`: this launch has helpers).
 template <int kMetric, bool kExact, bool kStage = false, bool kRegs = false, int kG = 0, bool kPipe = false,
-          bool kTrace = false>
+          bool kTrace = false, bool kHelp = false>
 __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, const WarpSmem& sm,
-                           uint32_t* stage_phase = nullptr) {
+                           uint32_t* stage_phase = nullptr, bool help = false) {
     const int lane = lane_id();
     const DeviceGraph& g = a.g;
     const uint32_t dim = g.dim;
@@ -2135,10 +2238,24 @@ __device__ void search_one(const SearchArgs& a, uint32_t qi, uint32_t slot, cons
         if (kTrace && a.tr.upper_only) {
             // The greedy descent alone: level 0 is not searched.
         } else if (kG > 0 && kPipe) {
-            overflowed = l0_team_lead<kG>(a, q, vs, sm, cur, ct, pc) && a.compact;
+            if (lane == 0) q.e[0].x |= kExplored;   // pop the cursor: the queue's only entry
+            q.hint = 1;
+            overflowed = l0_team_lead<kG>(a, q, vs, sm, cur, 0u, ct, pc) && a.compact;
         } else if (kPipe) {
-            overflowed = l0_search_pipelined<kMetric, kExact, kRegs>(a, q, vs, sm, qsq, cur, ct, pc, st) &&
+            Handover hand;
+            overflowed = l0_search_pipelined<kMetric, kExact, kRegs, kHelp>(a, q, vs, sm, qsq, cur, ct, pc, st, help,
+                                                                            hand) &&
                          a.compact;
+            if (kHelp && hand.first != kVidMask) {
+                HelpState h = {q, vs, ct, hand, qsq};
+                overflowed = help_lead<kHelpers>(a, threadIdx.x >> 5, h) && a.compact;
+                q.n = h.q.n;
+                q.lb = h.q.lb;
+                vs.global_used = h.vs.global_used;
+                vs.list_overflow = h.vs.list_overflow;
+                vs.list_n = h.vs.list_n;
+                ct = h.ct;
+            }
         } else {
             // Software pipeline: while one row is processed, the row descriptor and
             // then the neighbour ids of the entry that would be expanded next are
@@ -2302,7 +2419,8 @@ __global__ void __launch_bounds__(32, 24) search_plain_kernel(SearchArgs a) {
 // (3 x 256: 80 registers used, 24 warps), 96 (5 CTAs of at most 128 threads:
 // 20 warps) or 128 (4 CTAs of at most 128 threads: 16 warps; the pipelined
 // level-0 loop then holds the next expansion's first rows in registers).
-// (__maxnreg__ with the same counts measured slower.)
+// (__maxnreg__ with the same counts measured slower.) A warp that finds no query
+// left helps the CTA's last one (help_rows).
 constexpr int budget_threads(int budget) { return budget >= 96 ? 128 : 256; }
 constexpr int budget_min_blocks(int budget) {
     return budget == 64 ? 4 : (budget == 96 ? 5 : (budget == 128 ? 4 : 3));
@@ -2310,9 +2428,17 @@ constexpr int budget_min_blocks(int budget) {
 
 template <int kMetric, bool kExact, int kBudget, bool kStage = false, bool kPipe = false>
 __global__ void __launch_bounds__(budget_threads(kBudget), budget_min_blocks(kBudget))
-    search_persistent_kernel(SearchArgs a) {
+    search_persistent_kernel(const __grid_constant__ SearchArgs a) {
     extern __shared__ __align__(16) float smem[];
     const int warp = threadIdx.x >> 5;
+    // Only the 96- and 128-register kernels take helpers, and only CTAs of four warps.
+    constexpr bool kHelp = kPipe && !kStage;
+    const bool help = kHelp && blockDim.x == 32u * (kHelpers + 1) && !a.phase_cycles && (a.g.dim >> 4) <= kBlock;
+    HelpFlags* flags = reinterpret_cast<HelpFlags*>(smem);
+    if (help) {
+        if (threadIdx.x < 4) reinterpret_cast<uint32_t*>(smem)[threadIdx.x] = 0u;
+        __syncthreads();
+    }
     const uint32_t slot = blockIdx.x * (blockDim.x >> 5) + warp;
     const uint32_t stage_rows = kStage ? kStageRows : 0u;
     const WarpSmem sm = carve(smem + static_cast<size_t>(warp) * warp_smem_words(a.g.dim, a.cap, a.vh_bits,
@@ -2329,7 +2455,21 @@ __global__ void __launch_bounds__(budget_threads(kBudget), budget_min_blocks(kBu
         qi = __shfl_sync(kFull, qi, 0);
         if (qi >= a.nq) break;
         if (a.order) qi = __ldg(a.order + qi);
-        search_one<kMetric, kExact, kStage, kBudget == 128, 0, kPipe>(a, qi, slot, sm, &stage_phase);
+        search_one<kMetric, kExact, kStage, kBudget == 128, 0, kPipe, false, kHelp>(a, qi, slot, sm, &stage_phase,
+                                                                                   help);
+    }
+    if (help) {
+        uint32_t at = 0;
+        if (lane_id() == 0) {
+            at = atomicAdd(&flags->taken, 1u);
+            if (at == 0) flags->host = warp;
+            if (at == kHelpers) flags->quit = 1u;
+            __threadfence_block();
+            atomicAdd(&flags->idle, 1u);
+        }
+        at = __shfl_sync(kFull, at, 0);
+        if (at < kHelpers) help_rows<kMetric, kExact>(a, static_cast<int>(at));
+        else coop_barrier(kHelpers + 1);   // the last warp: the row warps leave
     }
     if (kStage) {
         __syncwarp();
