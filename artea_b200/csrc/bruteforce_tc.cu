@@ -24,8 +24,13 @@
 // 16 products, 32 times the unit of its FP32 accumulator), the FP32 chain of the
 // distance itself, and the rounding of sqrt (distances that are equal after it).
 // A query whose list does not fit, or an index or query whose norms leave the
-// range in which these bounds hold (not finite, or below 2^-50 or above 2^50),
-// goes to the FP32 scan.
+// range in which these bounds hold, goes to the FP32 scan: rows that are not
+// finite or whose nonzero norms leave [10^-9, 10^9], queries above 10^15, and for
+// dot below 2^-50, for cosine outside [10^-9, 10^9]. The lower limits keep what
+// FP32 sums of squares lose to underflow (elements below 2^-74: |q| and r_q fall
+// short by at most 2^-67 at 16,384 elements, R likewise) far below the 2^-14 of
+// |q||x| that E_q holds for the accumulation. Squared distances need none on the
+// query: there E_q holds 2^-14 of (|q| + |x|)^2, and |x| is at least 10^-9.
 //
 // What bounds it: at 1M x 128, 1,000 queries, k 100 the listing pass is 0.26 TFLOP
 // (0.16 ms at the measured FP16 rate) and takes 0.29 ms before hits, 0.47 ms with
@@ -620,11 +625,13 @@ __global__ void __launch_bounds__(256) bf_limit_kernel(const float* __restrict__
         const float g = (static_cast<float>(k_pad) / 16.0f + 32.0f) * 1.9073486e-6f;   // 2^-19 a step
         float e;
         bool safe = Q <= 1.0e15f;
+        // The lower limits on Q: see the top of the file.
         if (metric == ARTEA_GPU_COSINE) {
             e = rq + (Q + rq) * rel + g * Q;
             safe = Q >= 1.0e-9f && Q <= 1.0e9f;
         } else if (metric == ARTEA_GPU_DOT) {
             e = rq * X + (Q + rq) * R + g * Q * X;
+            safe = safe && Q >= 8.8817842e-16f;   // 2^-50
         } else {
             e = 2.0f * (rq * X + (Q + rq) * R) + g * (Q + X) * (Q + X);
         }

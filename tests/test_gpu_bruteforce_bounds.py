@@ -1,0 +1,45 @@
+"""Brute force where the tensor-core filter's bounds do not hold or its lists do
+not fit, and calls that must not depend on it: the words are the oracle's."""
+import numpy as np
+import pytest
+
+from artea_b200.router import DeviceIndex, vectors_only_graph
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _words(base, queries, k, metric):
+    ids, d = orc.bruteforce(base, queries, k, metric=metric)
+    return (d.view(np.uint32).astype(np.uint64) << np.uint64(32)) | ids.astype(np.uint64)
+
+
+def _normal(n, dim, seed):
+    return np.random.default_rng(seed).standard_normal((n, dim)).astype(np.float32)
+
+
+@pytest.mark.parametrize("metric", [0, 1, 2, 3])
+@pytest.mark.parametrize("exponent", [-9, -15, -17, -19, -21, -23])
+def test_queries_of_small_norm(metric, exponent):
+    """Squares of the elements underflow FP32 below about 1e-19."""
+    base, q = _normal(9000, 64, 1), _normal(20, 64, 2)
+    q *= np.float32(10.0 ** exponent)
+    q[::5] *= np.float32(1e-2)
+    idx = DeviceIndex(vectors_only_graph(), base)
+    np.testing.assert_array_equal(idx.bruteforce(q, 12, metric), _words(base, q, 12, metric))
+    idx.close()
+
+
+def test_dot_query_whose_norm_underflows():
+    """The nearest row is the one whose rounding to FP16 loses the most."""
+    base = np.full((9000, 128), 0.5, np.float32)
+    base[:2590:259] = 1.0 + 0.51 * 2.0 ** -10   # ten rows in ten tiles of 256
+    base[5000, 0::2] = 1.0 + 1.49 * 2.0 ** -10
+    base[5000, 1::2] = 1.0 + 0.49 * 2.0 ** -10
+    q = np.full((4, 128), 2.6e-23, np.float32)
+    q[:, 0] = 3e-23
+    idx = DeviceIndex(vectors_only_graph(), base)
+    got = idx.bruteforce(q, 10, 3)
+    assert (got[:, 0] & np.uint64(0xFFFFFFFF) == 5000).all()
+    np.testing.assert_array_equal(got, _words(base, q, 10, 3))
+    idx.close()
