@@ -488,7 +488,8 @@ __global__ void __launch_bounds__(256) bf_query_norms_kernel(const float* __rest
 }
 
 // Rows (vecs, or those of ids) to FP16, k_pad elements each (zeros past dim), 8
-// lanes a row, scaled by scale_from. Database rows: the residual norms' maxima
+// lanes a row, scaled by scale_from. vecs may be the caller's queries, which need
+// no more than a float's alignment: those are read one element at a time. Database rows: the residual norms' maxima
 // into res_max. Queries (qinfo): their residual norm.
 __global__ void __launch_bounds__(256) bf_round_kernel(const float* __restrict__ vecs, const uint32_t* __restrict__ ids,
                                                        const float* __restrict__ xsq, uint32_t n, uint32_t dim,
@@ -499,6 +500,7 @@ __global__ void __launch_bounds__(256) bf_round_kernel(const float* __restrict__
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const float scale = pow2_scale(sqrtf(__uint_as_float(scale_from->max_sq)));
     const float inv = 1.0f / scale;
+    const bool fours = (reinterpret_cast<uintptr_t>(vecs) & 15u) == 0u;
     uint32_t mres = 0, mrel = 0;
     for (uint32_t base = 4u * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < n; base += 4u * warps) {
         const uint32_t i = base + (lane >> 3);
@@ -510,7 +512,10 @@ __global__ void __launch_bounds__(256) bf_round_kernel(const float* __restrict__
 #pragma unroll 4
         for (uint32_t k = 4u * sub; k < k_pad; k += 32u) {   // dim is a multiple of 16: fours are whole
             if (!in) continue;
-            const float4 x = k < dim ? __ldg(reinterpret_cast<const float4*>(row + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k < dim)
+                x = fours ? __ldg(reinterpret_cast<const float4*>(row + k))
+                          : make_float4(__ldg(row + k), __ldg(row + k + 1u), __ldg(row + k + 2u), __ldg(row + k + 3u));
             const __half2 h0 = __floats2half2_rn(x.x * scale, x.y * scale), h1 = __floats2half2_rn(x.z * scale, x.w * scale);
             const float2 b0 = __half22float2(h0), b1 = __half22float2(h1);
             const float e0 = x.x - b0.x * inv, e1 = x.y - b0.y * inv, e2 = x.z - b1.x * inv, e3 = x.w - b1.y * inv;

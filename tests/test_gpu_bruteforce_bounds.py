@@ -43,3 +43,21 @@ def test_dot_query_whose_norm_underflows():
     assert (got[:, 0] & np.uint64(0xFFFFFFFF) == 5000).all()
     np.testing.assert_array_equal(got, _words(base, q, 10, 3))
     idx.close()
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+@pytest.mark.parametrize("metric", [0, 2, 3])
+def test_device_queries_at_any_float_offset(offset, metric):
+    import torch
+    base, q = _normal(9000, 80, 3), _normal(40, 80, 4)
+    idx = DeviceIndex(vectors_only_graph(), base)
+    flat = torch.zeros(q.size + 4, dtype=torch.float32, device="cuda")
+    view = flat[offset:offset + q.size]
+    view.copy_(torch.from_numpy(q.reshape(-1)))
+    assert view.data_ptr() % 16 == 4 * offset
+    want = _words(base, q, 10, metric)
+    for nq in (2, 40, 3):   # few queries, the filter, few queries through the filter
+        out = torch.zeros((nq, 10), dtype=torch.int64, device="cuda")
+        idx.bruteforce_device(view, nq, 10, metric, out)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want[:nq])
+    idx.close()
