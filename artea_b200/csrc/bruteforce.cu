@@ -33,6 +33,11 @@ constexpr uint32_t kBfMaxTopk = 1024;
 constexpr uint32_t kFilterRows = 8192;   // fewer rows: no filter
 constexpr uint32_t kFewRows = 1024;      // fewer rows: the scan
 constexpr uint32_t kFilterQueries = 4;   // fewer queries: bf_few, unless the index's rows are rounded already
+// Dynamic shared memory that the kernels are allowed (the scan's own variables take
+// less than 512 bytes of 227 KB, the merge sorts at most 16,384 keys). Fixed, since
+// the limit belongs to the function and calls of other sizes run at the same time.
+constexpr uint32_t kScanSmem = 227u * 1024u - 512u;
+constexpr uint32_t kMergeKeys = 16384;
 constexpr uint64_t kMaxKey = ~0ull;
 // CandidateEntry() (router/data_structures/candidate_entry.hpp:72-74): vid =
 // invalid_vertex_id (all ones), distance 0 -- the padding of batch rows whose
@@ -332,9 +337,9 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
     ScanFn fn = scan_kernel(metric);
     const uint32_t list_cap = next_pow2(topk + 2 * kBfThreads);
     const size_t smem = static_cast<size_t>(kBfQueries) * (list_cap * sizeof(uint64_t) + ix->dim * sizeof(float));
-    if (smem > 227u * 1024u) return fail(ARTEA_GPU_EINVAL, "brute-force tile exceeds shared memory (topk or dim too large)");
+    if (smem > kScanSmem) return fail(ARTEA_GPU_EINVAL, "brute-force tile exceeds shared memory (topk or dim too large)");
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
+                                  static_cast<int>(kScanSmem)));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn), kBfThreads,
                                                            smem));
@@ -348,7 +353,7 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
     uint32_t segments = std::max(1u, (want + tiles - 1) / tiles);
     segments = std::min(segments, std::max(1u, n_rows / std::min(4096u, std::max(512u, 32u * topk))));
     segments = std::min(segments, std::max(4096u / topk, 2u * static_cast<uint32_t>(dev_sms)));
-    segments = std::min(segments, std::max(1u, 16384u / topk));
+    segments = std::min(segments, std::max(1u, kMergeKeys / topk));
     const uint32_t seg_len = (n_rows + segments - 1) / segments;
     segments = (n_rows + seg_len - 1) / seg_len;
 
@@ -378,7 +383,8 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
         const uint32_t pow2 = next_pow2(segments * topk);
         const size_t msmem = static_cast<size_t>(pow2) * sizeof(uint64_t);
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(bf_merge_kernel),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(msmem));
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kMergeKeys * sizeof(uint64_t)));
         if (e == cudaSuccess) {
             bf_merge_kernel<<<nq, 256, msmem, st>>>(a.part, a.part_n, segments, topk, pow2, d_out);
             e = cudaGetLastError();

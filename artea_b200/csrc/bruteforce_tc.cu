@@ -72,6 +72,11 @@ constexpr uint32_t kWarpCols = kTileX / 2;   // columns of an epilogue warp
 constexpr uint32_t kHitBuffer = 192;      // hits a warp gathers before it appends them to the lists
 constexpr uint32_t kListCap = 4096;       // survivors of a query
 constexpr uint32_t kMaxGroups2 = 16384;   // group minima of a query
+// Dynamic shared memory that the kernels are allowed. The limit belongs to the
+// function, not to a call: one that followed a call's width could be lowered by
+// another thread between a call's setting it and its launch.
+constexpr uint32_t kFilterSmem = 190u * 1024u;
+constexpr uint32_t kRerankSmem = 160u * 1024u;
 constexpr uint32_t kSpin = 1u << 20;      // polls (each suspends for a while) before a wait counts as lost
 
 // Norms of the whole index (one per index, on the device).
@@ -1123,18 +1128,18 @@ int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uin
     const uint32_t chunks = k_pad / kChunkK;
     const bool resident = chunks <= kMaxResidentK;
     const uint32_t kept = 1024u + (resident ? chunks * kABytes : 0u), stage = kBBytes + (resident ? 0u : kABytes);
-    const uint32_t stages = std::min(kMaxStages, (190u * 1024u - kept) / stage);
+    const uint32_t stages = std::min(kMaxStages, (kFilterSmem - kept) / stage);
     // (At least half an SM's shared memory: one CTA an SM holds all its TMEM.)
     const uint32_t smem = std::max(117u * 1024u, kept + stages * stage);
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(bf_filter_kernel),
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFilterSmem)));
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(bf_limit_kernel),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxGroups2 * 4)));
     RerankFn rr = rerank_kernel(metric);
     const uint32_t rr_smem = kListCap * 12u + dim * 4u;
-    if (rr_smem > 227u * 1024u) return ARTEA_GPU_OK;
+    if (rr_smem > kRerankSmem) return ARTEA_GPU_OK;
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(rr), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(rr_smem)));
+                                  static_cast<int>(kRerankSmem)));
     for (uint32_t first = 0; first < nq; first += batch) {
         const uint32_t b = std::min(batch, nq - first);
         const float* qv = d_queries + static_cast<size_t>(first) * dim;

@@ -1,5 +1,7 @@
 """Brute force where the tensor-core filter's bounds do not hold or its lists do
 not fit, and calls that must not depend on it: the words are the oracle's."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -61,3 +63,39 @@ def test_device_queries_at_any_float_offset(offset, metric):
         idx.bruteforce_device(view, nq, 10, metric, out)
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint64), want[:nq])
     idx.close()
+
+
+def test_calls_of_other_widths_at_the_same_time():
+    """Each thread's calls on its own index and stream; widths, topk and row counts differ, so that
+    the kernels want other amounts of shared memory in each."""
+    import torch
+    jobs = []
+    for i, (n, dim, nq, k, metric) in enumerate([(9000, 64, 40, 10, 0), (8500, 960, 9, 100, 3), (9100, 400, 130, 1, 2),
+                                                 (3000, 128, 20, 300, 1)]):
+        base, q = _normal(n, dim, 10 + i), _normal(nq, dim, 20 + i)
+        jobs.append((DeviceIndex(vectors_only_graph(), base), torch.from_numpy(q).cuda(), nq, k, metric,
+                     _words(base, q, k, metric)))
+    wrong = []
+
+    def run(idx, dq, nq, k, metric, want):
+        try:
+            torch.cuda.set_device(0)
+            s = torch.cuda.Stream()
+            out = torch.zeros((nq, k), dtype=torch.int64, device="cuda")
+            s.wait_stream(torch.cuda.current_stream())
+            for _ in range(60):
+                idx.bruteforce_device(dq, nq, k, metric, out, stream=s.cuda_stream)
+                if not np.array_equal(out.cpu().numpy().view(np.uint64), want):
+                    wrong.append((nq, k, metric))
+        except Exception as e:   # a refused launch
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=run, args=j) for j in jobs]
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(120)
+    assert not wrong, wrong[:4]
+    for j in jobs:
+        j[0].close()
