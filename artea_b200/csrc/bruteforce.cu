@@ -416,6 +416,7 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
     }
     int dev_sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ix->device));
+    work.start(st);
     const uint32_t* subset = use_subset ? d_subset : nullptr;
     // The tensor-core filter reads every row twice in FP16 and pays a rounding pass
     // over the rows (once an index, or on every call for a subset); bf_few reads them
@@ -436,10 +437,13 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
                 if (int rc = scan(ix, metric, d_queries + static_cast<size_t>(q) * ix->dim, 1, topk, subset, n_rows,
                                   d_out + static_cast<size_t>(q) * topk, work, dev_sms, st))
                     return rc;
+            work.waited();
             return ARTEA_GPU_OK;
         }
     }
-    return scan(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st);
+    if (int rc = scan(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st)) return rc;
+    work.waited();
+    return ARTEA_GPU_OK;
 }
 
 // Centroid of the bucket's rows (hierarchical_graph_compactor.hpp:261-300):
@@ -571,6 +575,7 @@ int artea_gpu_centroid_entry(const artea_gpu_index* index, int metric, const uin
     uint32_t* d_bucket = bucket ? reinterpret_cast<uint32_t*>(p + partial_bytes + centroid_bytes + 16) : nullptr;
     if (bucket && cudaMemcpy(d_bucket, bucket, sizeof(uint32_t) * n, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(ARTEA_GPU_ECUDA, "bucket upload failed");
+    work.start(nullptr);
     centroid_partial_kernel<<<dim3(blocks, (index->dim + 31) / 32), 32>>>(index->d_vecs, index->dim, d_bucket, rows,
                                                                          per_block, d_partial);
     centroid_final_kernel<<<(index->dim + 31) / 32, 32>>>(d_partial, blocks, index->dim, rows, d_centroid);

@@ -17,18 +17,23 @@ BfCache* bf_cache_create(int device, const float* d_xsq, uint32_t n, int sms);  
 void bf_cache_destroy(BfCache* c);
 
 // A call's device workspace: the device's, unless another thread's call holds it.
-// Slot 0: the host entry points' copies; slot 1: everything else.
+// Slot 0: the host entry points' copies; slot 1: everything else. A call that ends
+// early (an error) may leave kernels on its stream: they are waited for before the
+// memory goes to another call.
 constexpr size_t kBfKeepBytes = 256u << 20;   // no larger one is kept (per slot)
 struct BfWork {
     explicit BfWork(const artea_gpu_index* ix);
     ~BfWork();
     BfWork(const BfWork&) = delete;
     BfWork& operator=(const BfWork&) = delete;
+    void start(cudaStream_t st) { stream = st, running = true; }   // kernels may be in flight on st
+    void waited() { running = false; }
     // At least bytes, valid until the slot's next get() or the end.
     int get(int slot, size_t bytes, unsigned char** p);
 
     BfPool* pool;
-    bool held = false;
+    bool held = false, running = false;
+    cudaStream_t stream = nullptr;
     unsigned char* own[2] = {};
 };
 

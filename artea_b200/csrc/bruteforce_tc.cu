@@ -994,6 +994,10 @@ int BfWork::get(int slot, size_t bytes, unsigned char** p) {
 }
 
 BfWork::~BfWork() {
+    if (running) {
+        cudaStreamSynchronize(stream);
+        cudaGetLastError();
+    }
     for (auto& p : own) dev_free(p);
     if (held) {
         for (int i = 0; i < 2; ++i) {   // a large workspace is not kept

@@ -99,3 +99,25 @@ def test_calls_of_other_widths_at_the_same_time():
     assert not wrong, wrong[:4]
     for j in jobs:
         j[0].close()
+
+
+def test_a_call_that_is_refused_leaves_the_workspace_to_the_next():
+    """Waiting for a stream that is being captured is refused, in the middle of a call."""
+    import torch
+    from cuda.bindings import runtime as rt
+    base, q = _normal(9000, 64, 5), _normal(30, 64, 6)
+    idx = DeviceIndex(vectors_only_graph(), base)
+    want = _words(base, q, 10, 0)
+    dq = torch.from_numpy(q).cuda()
+    out = torch.zeros((30, 10), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    for nq in (30, 2):
+        s = torch.cuda.Stream()
+        assert rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed)[0] == 0
+        with pytest.raises(RuntimeError):
+            idx.bruteforce_device(dq, nq, 10, 0, out, stream=s.cuda_stream)
+        rt.cudaStreamEndCapture(s.cuda_stream)
+        rt.cudaGetLastError()
+        idx.bruteforce_device(dq, nq, 10, 0, out[:nq])
+        np.testing.assert_array_equal(out[:nq].cpu().numpy().view(np.uint64), want[:nq])
+    idx.close()
