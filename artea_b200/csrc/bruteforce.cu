@@ -331,13 +331,17 @@ ScanFn scan_kernel(int metric) {
     }
 }
 
+uint32_t scan_list_cap(uint32_t topk) { return next_pow2(topk + 2 * kBfThreads); }
+size_t scan_smem(uint32_t dim, uint32_t topk) {
+    return static_cast<size_t>(kBfQueries) * (scan_list_cap(topk) * sizeof(uint64_t) + dim * sizeof(float));
+}
+
 // The FP32 scan of rows [0, n_rows) (d_subset null) or d_subset's; waits.
 int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
          const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int dev_sms, cudaStream_t st) {
     ScanFn fn = scan_kernel(metric);
-    const uint32_t list_cap = next_pow2(topk + 2 * kBfThreads);
-    const size_t smem = static_cast<size_t>(kBfQueries) * (list_cap * sizeof(uint64_t) + ix->dim * sizeof(float));
-    if (smem > kScanSmem) return fail(ARTEA_GPU_EINVAL, "brute-force tile exceeds shared memory (topk or dim too large)");
+    const uint32_t list_cap = scan_list_cap(topk);
+    const size_t smem = scan_smem(ix->dim, topk);
     CUDA_TRY(cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(kScanSmem)));
     int per_sm = 0;
@@ -414,6 +418,10 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
         CUDA_TRY(cudaStreamSynchronize(st));
         return ARTEA_GPU_OK;
     }
+    // Sizes that the scan cannot take are refused whatever path the call would go
+    // first: any of them may hand queries on to the scan.
+    if (scan_smem(ix->dim, topk) > kScanSmem)
+        return fail(ARTEA_GPU_EINVAL, "brute-force tile exceeds shared memory (topk or dim too large)");
     int dev_sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ix->device));
     work.start(st);

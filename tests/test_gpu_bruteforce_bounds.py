@@ -5,6 +5,7 @@ import threading
 import numpy as np
 import pytest
 
+from artea_b200._native import ArteaGpuError
 from artea_b200.router import DeviceIndex, vectors_only_graph
 from oracle import oracle as orc
 
@@ -120,4 +121,15 @@ def test_a_call_that_is_refused_leaves_the_workspace_to_the_next():
         rt.cudaGetLastError()
         idx.bruteforce_device(dq, nq, 10, 0, out[:nq])
         np.testing.assert_array_equal(out[:nq].cpu().numpy().view(np.uint64), want[:nq])
+    idx.close()
+
+
+@pytest.mark.parametrize("nq", [2, 5])
+@pytest.mark.parametrize("n,dim,topk", [(8300, 3200, 1024), (8300, 6752, 256)])
+def test_tiles_above_the_scans_shared_memory_are_refused(n, dim, topk, nq):
+    """8 queries' lists and rows in 227 KB: the last dims that fit are 3,152 at topk 1,024 and 6,224 at 256."""
+    base, q = _normal(n, dim, 7), _normal(nq, dim, 8)
+    idx = DeviceIndex(vectors_only_graph(), base)
+    with pytest.raises(ArteaGpuError, match="EINVAL"):
+        idx.bruteforce(q, topk, 0)
     idx.close()
