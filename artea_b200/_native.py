@@ -146,6 +146,7 @@ SIGNATURES = {
     "artea_gpu_router_set_phase_buffer": (c_int, [c_void_p, c_void_p]),
     "artea_gpu_router_set_early_stop": (c_int, [c_void_p, c_void_p, c_uint32]),
     "artea_gpu_bruteforce": (c_int, [c_void_p, c_int, c_void_p, c_uint32, c_uint32, c_void_p, c_uint32, c_void_p]),
+    "artea_gpu_bruteforce_last": (c_int, [c_void_p, POINTER(c_uint32), POINTER(c_uint32)]),
     "artea_gpu_centroid_entry": (c_int, [c_void_p, c_int, c_void_p, c_uint32, c_void_p]),
     "artea_gpu_bruteforce_device": (c_int, [c_void_p, c_int, c_void_p, c_uint32, c_uint32, c_void_p, c_uint32,
                                             c_void_p, c_void_p]),

@@ -107,6 +107,7 @@ struct BfArgs {
     const uint32_t* __restrict__ subset;   // null: rows [0, n_rows)
     uint32_t n_rows;
     const float* __restrict__ queries;
+    const uint32_t* __restrict__ which;    // nq queries' rows in queries and out (null: 0..nq-1)
     uint32_t nq;
     uint32_t k;
     uint32_t seg_len;                      // rows per segment (blockIdx.y)
@@ -133,7 +134,9 @@ __global__ void __launch_bounds__(kBfThreads) bf_scan_kernel(BfArgs a) {
     const uint32_t dim = a.dim;
     for (uint32_t i = tid; i < kBfQueries * dim; i += kBfThreads) {
         const uint32_t qi = i / dim;
-        qs[i] = qi < nqt ? a.queries[static_cast<size_t>(q0 + qi) * dim + (i - qi * dim)] : 0.0f;
+        float v = 0.0f;
+        if (qi < nqt) v = a.queries[static_cast<size_t>(a.which ? a.which[q0 + qi] : q0 + qi) * dim + (i - qi * dim)];
+        qs[i] = v;
     }
     if (tid < kBfQueries) {
         cnt[tid] = 0;
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(kBfThreads) bf_scan_kernel(BfArgs a) {
         const uint64_t* l = lists + static_cast<size_t>(qi) * a.list_cap;
         const uint32_t n = cnt[qi];
         if (a.segments == 1) {
-            uint64_t* o = a.out + static_cast<size_t>(q0 + qi) * a.k;
+            uint64_t* o = a.out + static_cast<size_t>(a.which ? a.which[q0 + qi] : q0 + qi) * a.k;
             for (uint32_t i = tid; i < a.k; i += kBfThreads) o[i] = i < n ? key_word(l[i]) : kDefaultEntryWord;
         } else {
             uint64_t* o = a.part + (static_cast<size_t>(q0 + qi) * a.segments + blockIdx.y) * a.k;
@@ -286,7 +289,8 @@ __global__ void __launch_bounds__(kBfThreads) bf_scan_kernel(BfArgs a) {
 // One CTA per query: the best k of its segments' sorted key lists.
 __global__ void __launch_bounds__(256) bf_merge_kernel(const uint64_t* __restrict__ part,
                                                        const uint32_t* __restrict__ part_n, uint32_t segments,
-                                                       uint32_t k, uint32_t pow2, uint64_t* __restrict__ out) {
+                                                       uint32_t k, uint32_t pow2, const uint32_t* __restrict__ which,
+                                                       uint64_t* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char bf_smem[];
     uint64_t* keys = reinterpret_cast<uint64_t*>(bf_smem);   // pow2 >= segments * k
     const uint32_t q = blockIdx.x;
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(256) bf_merge_kernel(const uint64_t* __restric
             __syncthreads();
         }
     }
-    uint64_t* o = out + static_cast<size_t>(q) * k;
+    uint64_t* o = out + static_cast<size_t>(which ? which[q] : q) * k;
     for (uint32_t i = threadIdx.x; i < k; i += blockDim.x)
         o[i] = keys[i] != kMaxKey ? key_word(keys[i]) : kDefaultEntryWord;
 }
@@ -336,9 +340,13 @@ size_t scan_smem(uint32_t dim, uint32_t topk) {
     return static_cast<size_t>(kBfQueries) * (scan_list_cap(topk) * sizeof(uint64_t) + dim * sizeof(float));
 }
 
-// The FP32 scan of rows [0, n_rows) (d_subset null) or d_subset's; waits.
+// The FP32 scan of rows [0, n_rows) (d_subset null) or d_subset's, for nq queries or
+// those of `which` (in one launch: a query at a time cost a launch, a wait and a
+// pass over the rows each, eight of which a CTA does at once); waits.
 int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t nq, uint32_t topk,
-         const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int dev_sms, cudaStream_t st) {
+         const uint32_t* d_subset, uint32_t n_rows, uint64_t* d_out, BfWork& work, int dev_sms, cudaStream_t st,
+         const std::vector<uint32_t>* which = nullptr) {
+    if (which) nq = static_cast<uint32_t>(which->size());
     ScanFn fn = scan_kernel(metric);
     const uint32_t list_cap = scan_list_cap(topk);
     const size_t smem = scan_smem(ix->dim, topk);
@@ -374,13 +382,20 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
     a.segments = segments;
     a.list_cap = list_cap;
     a.out = d_out;
-    if (segments > 1) {
-        const size_t keys = sizeof(uint64_t) * static_cast<size_t>(nq) * segments * topk;
+    if (segments > 1 || which) {
+        const size_t keys = segments > 1 ? sizeof(uint64_t) * static_cast<size_t>(nq) * segments * topk : 0;
+        const size_t counts = segments > 1 ? sizeof(uint32_t) * static_cast<size_t>(nq) * segments : 0;
         unsigned char* p = nullptr;
-        if (int rc = work.get(1, keys + sizeof(uint32_t) * static_cast<size_t>(nq) * segments, &p)) return rc;
+        if (int rc = work.get(1, keys + counts + (which ? sizeof(uint32_t) * nq : 0), &p)) return rc;
         a.part = reinterpret_cast<uint64_t*>(p);
         a.part_n = reinterpret_cast<uint32_t*>(p + keys);
+        if (which) {
+            a.which = reinterpret_cast<uint32_t*>(p + keys + counts);
+            CUDA_TRY(cudaMemcpyAsync(p + keys + counts, which->data(), sizeof(uint32_t) * nq, cudaMemcpyHostToDevice, st));
+        }
     }
+    ix->bf->last_scanned += nq;
+    ++ix->bf->last_scans;
     fn<<<dim3(tiles, segments), kBfThreads, smem, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && segments > 1) {
@@ -390,7 +405,7 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(kMergeKeys * sizeof(uint64_t)));
         if (e == cudaSuccess) {
-            bf_merge_kernel<<<nq, 256, msmem, st>>>(a.part, a.part_n, segments, topk, pow2, d_out);
+            bf_merge_kernel<<<nq, 256, msmem, st>>>(a.part, a.part_n, segments, topk, pow2, a.which, d_out);
             e = cudaGetLastError();
         }
     }
@@ -425,6 +440,8 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
     int dev_sms = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ix->device));
     work.start(st);
+    ix->bf->last_scanned = 0;
+    ix->bf->last_scans = 0;
     const uint32_t* subset = use_subset ? d_subset : nullptr;
     // The tensor-core filter reads every row twice in FP16 and pays a rounding pass
     // over the rows (once an index, or on every call for a subset); bf_few reads them
@@ -440,10 +457,9 @@ int bruteforce_impl(const artea_gpu_index* ix, int metric, const float* d_querie
         if (int rc = filter ? bf_tensor(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &used, &redo)
                             : bf_few(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &used, &redo))
             return rc;
-        if (used && redo.size() <= 64) {
-            for (const uint32_t q : redo)
-                if (int rc = scan(ix, metric, d_queries + static_cast<size_t>(q) * ix->dim, 1, topk, subset, n_rows,
-                                  d_out + static_cast<size_t>(q) * topk, work, dev_sms, st))
+        if (used && redo.size() < nq) {
+            if (!redo.empty())
+                if (int rc = scan(ix, metric, d_queries, nq, topk, subset, n_rows, d_out, work, dev_sms, st, &redo))
                     return rc;
             work.waited();
             return ARTEA_GPU_OK;
@@ -522,6 +538,13 @@ int artea_gpu_bruteforce_device(const artea_gpu_index* index, int metric, const 
     BfWork work(index);
     return bruteforce_impl(index, metric, d_queries, nq, topk, d_subset != nullptr, d_subset, n_subset, d_out, work,
                            static_cast<cudaStream_t>(stream));
+}
+
+int artea_gpu_bruteforce_last(const artea_gpu_index* index, uint32_t* scanned, uint32_t* scans) {
+    if (!index || !scanned || !scans) return fail(ARTEA_GPU_EINVAL, "null argument");
+    *scanned = index->bf->last_scanned;
+    *scans = index->bf->last_scans;
+    return ARTEA_GPU_OK;
 }
 
 int artea_gpu_bruteforce(const artea_gpu_index* index, int metric, const float* queries, uint32_t nq, uint32_t topk,

@@ -1,18 +1,43 @@
 // Brute force through the tensor cores (bruteforce_tc.cu), used by bruteforce.cu.
 #pragma once
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 struct artea_gpu_index;
 
 namespace artea_gpu {
 
-struct BfCache;
 struct BfPool;
+
+// Norms of the whole index (one per index, on the device).
+struct BfStats {
+    uint32_t max_sq;     // largest x.x (float bits; sums of squares order as unsigned)
+    uint32_t min_sq;     // smallest nonzero x.x
+    uint32_t bad;        // some x.x is not finite
+    uint32_t max_res;    // largest |x - fp16(x)| (float bits)
+    uint32_t max_rel;    // largest |x - fp16(x)| / |x|
+    uint32_t pad[3];
+};
+
+// The state an index keeps for brute force: norms, and the rounded rows once a call
+// wanted them.
+struct BfCache {
+    int device = 0;
+    std::mutex mu;                  // rows
+    bool norms_ready = false, rows_ready = false, rows_failed = false;
+    BfStats norms = {};             // host copy
+    BfStats* d_norms = nullptr;
+    __half* d_rows = nullptr;
+    // The last call (artea_gpu_bruteforce_last): queries that the scan answered, its launches.
+    std::atomic<uint32_t> last_scanned{0}, last_scans{0};
+};
 BfCache* bf_cache_create(int device, const float* d_xsq, uint32_t n, int sms);   // d_xsq: x.x of every row
 void bf_cache_destroy(BfCache* c);
 

@@ -79,16 +79,6 @@ constexpr uint32_t kFilterSmem = 190u * 1024u;
 constexpr uint32_t kRerankSmem = 160u * 1024u;
 constexpr uint32_t kSpin = 1u << 20;      // polls (each suspends for a while) before a wait counts as lost
 
-// Norms of the whole index (one per index, on the device).
-struct BfStats {
-    uint32_t max_sq;     // largest x.x (float bits; sums of squares order as unsigned)
-    uint32_t min_sq;     // smallest nonzero x.x
-    uint32_t bad;        // some x.x is not finite
-    uint32_t max_res;    // largest |x - fp16(x)| (float bits)
-    uint32_t max_rel;    // largest |x - fp16(x)| / |x|
-    uint32_t pad[3];
-};
-
 struct FilterArgs {
     const float* a;          // rows: A, at whole tiles (infinite past n_rows)
     const float* b;          // rows: B (null: 1)
@@ -910,17 +900,6 @@ bool encode(CUtensorMap* map, void* base, uint64_t rows, uint32_t k_pad, uint32_
 }
 
 }  // namespace
-
-// The state an index keeps for brute force: norms, and the rounded rows once a call
-// wanted them.
-struct BfCache {
-    int device = 0;
-    std::mutex mu;                  // rows
-    bool norms_ready = false, rows_ready = false, rows_failed = false;
-    BfStats norms = {};             // host copy
-    BfStats* d_norms = nullptr;
-    __half* d_rows = nullptr;
-};
 
 // A device's workspace, shared by its indexes and freed with the last of them: a
 // first call on a new index would otherwise pay its allocation. The call that holds

@@ -152,6 +152,12 @@ class DeviceIndex:
                                                         topk, nat.ptr(d_subset), n_subset, nat.ptr(d_out),
                                                         ctypes.c_void_p(stream or None)))
 
+    def last_bruteforce(self) -> dict:
+        """Of the last brute-force call: queries that the FP32 scan answered, and its launches."""
+        n, s = ctypes.c_uint32(), ctypes.c_uint32()
+        nat.check(nat.lib().artea_gpu_bruteforce_last(self.handle, ctypes.byref(n), ctypes.byref(s)))
+        return {"scanned": n.value, "scans": s.value}
+
     def close(self) -> None:
         if getattr(self, "_h", None) is not None:
             nat.lib().artea_gpu_index_destroy(self._h)

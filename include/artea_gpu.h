@@ -316,6 +316,11 @@ int artea_gpu_bruteforce_device(const artea_gpu_index* index, int metric, const 
                                 uint32_t topk, const uint32_t* d_subset, uint32_t n_subset, uint64_t* d_out,
                                 void* stream);
 
+/* How the last brute-force call on the index ran: the queries that the FP32 scan
+ * answered (all of them where no faster path applies; else those whose candidate
+ * lists did not fit) and the scan's launches. Measurement only. */
+int artea_gpu_bruteforce_last(const artea_gpu_index* index, uint32_t* scanned, uint32_t* scans);
+
 /* The compactor's entry point (hierarchical_graph_compactor.hpp:261-327,
  * _compute_entry_point_vid): the centroid of bucket's vectors (double sums,
  * rounded to float), then the bucket vid nearest to it under metric (the

@@ -133,3 +133,19 @@ def test_tiles_above_the_scans_shared_memory_are_refused(n, dim, topk, nq):
     with pytest.raises(ArteaGpuError, match="EINVAL"):
         idx.bruteforce(q, topk, 0)
     idx.close()
+
+
+@pytest.mark.parametrize("metric", [0, 1, 2, 3])
+@pytest.mark.parametrize("n,nq", [(9000, 2), (9000, 24), (9000, 300), (40000, 13)])
+def test_queries_whose_lists_overflow_are_scanned_together(n, nq, metric):
+    """Half of the queries are nearest to one row that is there 6,000 times: more than a list holds."""
+    rng = np.random.default_rng(n + nq)
+    base = rng.integers(-8, 9, (n, 48)).astype(np.float32)
+    base[100:6100] = 20.0
+    q = rng.integers(-8, 9, (nq, 48)).astype(np.float32)
+    q[::2] = 19.0 + rng.integers(0, 3, (len(q[::2]), 48))
+    idx = DeviceIndex(vectors_only_graph(), base)
+    np.testing.assert_array_equal(idx.bruteforce(q, 30, metric), _words(base, q, 30, metric))
+    last = idx.last_bruteforce()
+    assert last["scans"] == 1 and len(q[::2]) <= last["scanned"] < nq, last
+    idx.close()
