@@ -96,8 +96,8 @@ struct FilterArgs {
     uint32_t* count;         // nq
     uint2* list;             // nq x kListCap: {row, v}
     int* error;
-    const BfStats* xs;       // scales of the rows and the queries
-    const BfStats* qs;
+    const BfStats* xs;       // scale of the rows
+    const float4* qinfo;     // queries: norm, residual norm, 1 / scale
     float sign;              // factor of q.x in v: -2 or -1
 };
 
@@ -323,8 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf_filter_kernel(const __grid_con
         const uint32_t q = qt * kTileQ + 32u * quadrant + lane;
         const bool valid = q < a.nq;
         const bool collect = a.limit != nullptr;
-        const float beta = a.sign / pow2_scale(sqrtf(__uint_as_float(a.xs->max_sq))) /
-                           pow2_scale(sqrtf(__uint_as_float(a.qs->max_sq)));
+        const float beta = a.sign / pow2_scale(sqrtf(__uint_as_float(a.xs->max_sq))) * (valid ? a.qinfo[q].z : 0.0f);
         const f32x2 beta2 = pack2(beta, beta);
         const float limit = collect && valid ? a.limit[q] : -INFINITY;
         float m[32];
@@ -467,35 +466,45 @@ __global__ void __launch_bounds__(256) bf_norms_kernel(const float* __restrict__
     }
 }
 
-// Queries: norm and the batch's largest x.x (one warp a query).
-__global__ void __launch_bounds__(256) bf_query_norms_kernel(const float* __restrict__ q, uint32_t n, uint32_t dim,
-                                                             float4* __restrict__ qinfo, BfStats* stats) {
+// Queries to FP16, k_pad elements each (zeros past dim), one warp a query, with its
+// norm, residual norm and 1 / scale. Each has the scale of its own norm: with one for
+// the batch, one query of 10^12 times the others' norm rounded those to nothing and
+// sent them to the scan. The caller's queries need no more than a float's alignment.
+__global__ void __launch_bounds__(256) bf_round_queries_kernel(const float* __restrict__ q, uint32_t n, uint32_t dim,
+                                                               uint32_t k_pad, __half* __restrict__ out,
+                                                               float4* __restrict__ qinfo) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= n) return;   // warp-uniform
+    const float* row = q + static_cast<size_t>(i) * dim;
     float sq = 0.0f;
-    for (uint32_t k = lane; k < dim; k += 32) sq = fmaf(q[static_cast<size_t>(i) * dim + k], q[static_cast<size_t>(i) * dim + k], sq);
+    for (uint32_t k = lane; k < dim; k += 32) sq = fmaf(row[k], row[k], sq);
     for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
-    if (lane == 0) {
-        qinfo[i] = make_float4(sqrtf(sq) * 1.00001f, 0.0f, 0.0f, 0.0f);
-        if (isfinite(sq)) atomicMax(&stats->max_sq, __float_as_uint(sq));   // others go to the scan
+    const float norm = sqrtf(sq), scale = pow2_scale(norm), inv = 1.0f / scale;
+    float res = 0.0f;
+    __half2* o = reinterpret_cast<__half2*>(out + static_cast<size_t>(i) * k_pad);
+    for (uint32_t k = 2u * lane; k < k_pad; k += 64) {
+        const float x = k < dim ? row[k] : 0.0f, y = k < dim ? row[k + 1u] : 0.0f;   // dim is even
+        const __half2 h = __floats2half2_rn(x * scale, y * scale);
+        const float2 b = __half22float2(h);
+        const float e0 = x - b.x * inv, e1 = y - b.y * inv;
+        res = fmaf(e0, e0, fmaf(e1, e1, res));
+        o[k / 2u] = h;
     }
+    for (int off = 16; off > 0; off >>= 1) res += __shfl_xor_sync(0xffffffffu, res, off);
+    if (lane == 0) qinfo[i] = make_float4(norm * 1.00001f, sqrtf(res) * 1.00001f, inv, 0.0f);
 }
 
 // Rows (vecs, or those of ids) to FP16, k_pad elements each (zeros past dim), 8
-// lanes a row, scaled by scale_from. vecs may be the caller's queries, which need
-// no more than a float's alignment: those are read one element at a time. Database rows: the residual norms' maxima
-// into res_max. Queries (qinfo): their residual norm.
+// lanes a row, scaled by scale_from; the residual norms' maxima into res_max.
 __global__ void __launch_bounds__(256) bf_round_kernel(const float* __restrict__ vecs, const uint32_t* __restrict__ ids,
                                                        const float* __restrict__ xsq, uint32_t n, uint32_t dim,
                                                        uint32_t k_pad, const BfStats* scale_from,
-                                                       __half* __restrict__ out, BfStats* res_max,
-                                                       float4* __restrict__ qinfo) {
+                                                       __half* __restrict__ out, BfStats* res_max) {
     const uint32_t lane = threadIdx.x & 31u, sub = lane & 7u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const float scale = pow2_scale(sqrtf(__uint_as_float(scale_from->max_sq)));
     const float inv = 1.0f / scale;
-    const bool fours = (reinterpret_cast<uintptr_t>(vecs) & 15u) == 0u;
     uint32_t mres = 0, mrel = 0;
     for (uint32_t base = 4u * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < n; base += 4u * warps) {
         const uint32_t i = base + (lane >> 3);
@@ -507,10 +516,7 @@ __global__ void __launch_bounds__(256) bf_round_kernel(const float* __restrict__
 #pragma unroll 4
         for (uint32_t k = 4u * sub; k < k_pad; k += 32u) {   // dim is a multiple of 16: fours are whole
             if (!in) continue;
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < dim)
-                x = fours ? __ldg(reinterpret_cast<const float4*>(row + k))
-                          : make_float4(__ldg(row + k), __ldg(row + k + 1u), __ldg(row + k + 2u), __ldg(row + k + 3u));
+            const float4 x = k < dim ? __ldg(reinterpret_cast<const float4*>(row + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             const __half2 h0 = __floats2half2_rn(x.x * scale, x.y * scale), h1 = __floats2half2_rn(x.z * scale, x.w * scale);
             const float2 b0 = __half22float2(h0), b1 = __half22float2(h1);
             const float e0 = x.x - b0.x * inv, e1 = x.y - b0.y * inv, e2 = x.z - b1.x * inv, e3 = x.w - b1.y * inv;
@@ -523,21 +529,17 @@ __global__ void __launch_bounds__(256) bf_round_kernel(const float* __restrict__
 #pragma unroll
         for (int off = 4; off > 0; off >>= 1) res += __shfl_xor_sync(0xffffffffu, res, off);
         const float r = sqrtf(res) * 1.00001f;
-        if (qinfo) {
-            if (in && sub == 0u) qinfo[i].y = r;
-        } else if (in) {
+        if (in) {
             const float norm = sqrtf(xsq[vid]);
             mres = max(mres, __float_as_uint(r));
             if (norm > 0.0f) mrel = max(mrel, __float_as_uint(r / norm * 1.00001f));
         }
     }
-    if (!qinfo) {
-        mres = __reduce_max_sync(0xffffffffu, mres);
-        mrel = __reduce_max_sync(0xffffffffu, mrel);
-        if (lane == 0) {
-            atomicMax(&res_max->max_res, mres);
-            atomicMax(&res_max->max_rel, mrel);
-        }
+    mres = __reduce_max_sync(0xffffffffu, mres);
+    mrel = __reduce_max_sync(0xffffffffu, mrel);
+    if (lane == 0) {
+        atomicMax(&res_max->max_res, mres);
+        atomicMax(&res_max->max_rel, mrel);
     }
 }
 
@@ -1011,7 +1013,7 @@ bool bf_prepare(const artea_gpu_index* ix, bool want_rows, int sms, cudaStream_t
             return false;
         }
         bf_round_kernel<<<sms * 8, 256, 0, st>>>(ix->d_vecs, nullptr, ix->d_xsq, ix->nvecs, ix->dim, k_pad, c->d_norms,
-                                                 c->d_rows, c->d_norms, nullptr);
+                                                 c->d_rows, c->d_norms);
         if (cudaStreamSynchronize(st) != cudaSuccess) {   // other streams may use them next
             dev_free(c->d_rows);
             c->rows_failed = true;
@@ -1074,7 +1076,7 @@ int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uin
         return p;
     };
     const size_t o_q = take(static_cast<size_t>(batch) * k_pad * 2), o_info = take(sizeof(float4) * batch);
-    const size_t o_qs = take(sizeof(BfStats)), o_min = take(sizeof(float) * batch * static_cast<size_t>(most));
+    const size_t o_min = take(sizeof(float) * batch * static_cast<size_t>(most));
     const size_t o_lim = take(sizeof(float) * batch), o_cnt = take(sizeof(uint32_t) * batch);
     const size_t o_spread = take(sizeof(float) * batch);
     const size_t o_list = take(sizeof(uint2) * batch * static_cast<size_t>(kListCap));
@@ -1087,7 +1089,6 @@ int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uin
     if (work.get(1, at, &base) != ARTEA_GPU_OK) return ARTEA_GPU_OK;   // the scan needs less
     auto* q16 = reinterpret_cast<__half*>(base + o_q);
     auto* info = reinterpret_cast<float4*>(base + o_info);
-    auto* qs = reinterpret_cast<BfStats*>(base + o_qs);
     auto* rs = reinterpret_cast<BfStats*>(base + o_rs);
     auto* d_redo = reinterpret_cast<uint32_t*>(base + o_redo);   // count, indices..., error word last
     auto* col_a = reinterpret_cast<float*>(base + o_a);
@@ -1101,7 +1102,7 @@ int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uin
         x16 = reinterpret_cast<__half*>(base + o_rows);
         CUDA_TRY(cudaMemsetAsync(rs, 0, sizeof(BfStats), st));
         bf_round_kernel<<<sms * 8, 256, 0, st>>>(ix->d_vecs, d_subset, ix->d_xsq, n_rows, dim, k_pad, c->d_norms, x16,
-                                                 rs, nullptr);
+                                                 rs);
         res = rs;
     }
     bf_ab_kernel<<<(n_pad + 255) / 256, 256, 0, st>>>(d_subset, ix->d_xsq, n_rows, n_pad, metric, col_a, col_b);
@@ -1127,9 +1128,7 @@ int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uin
         const uint32_t b = std::min(batch, nq - first);
         const float* qv = d_queries + static_cast<size_t>(first) * dim;
         shape(b, &rg, &per_flush, &groups);
-        CUDA_TRY(cudaMemsetAsync(qs, 0, sizeof(BfStats), st));
-        bf_query_norms_kernel<<<(b + 7) / 8, 256, 0, st>>>(qv, b, dim, info, qs);
-        bf_round_kernel<<<(b + 31) / 32, 256, 0, st>>>(qv, nullptr, nullptr, b, dim, k_pad, qs, q16, nullptr, info);
+        bf_round_queries_kernel<<<(b + 7) / 8, 256, 0, st>>>(qv, b, dim, k_pad, q16, info);
         if (!encode(&map_q, q16, b, k_pad, kTileQ)) return fail(ARTEA_GPU_ECUDA, "brute force: query tensor map");
         FilterArgs f;
         std::memset(&f, 0, sizeof(f));
@@ -1149,7 +1148,7 @@ int bf_tensor(const artea_gpu_index* ix, int metric, const float* d_queries, uin
         f.list = reinterpret_cast<uint2*>(base + o_list);
         f.error = d_error;
         f.xs = c->d_norms;
-        f.qs = qs;
+        f.qinfo = info;
         f.sign = metric == ARTEA_GPU_COSINE || metric == ARTEA_GPU_DOT ? -1.0f : -2.0f;
         float* limit = reinterpret_cast<float*>(base + o_lim);
         float* spread = reinterpret_cast<float*>(base + o_spread);

@@ -149,3 +149,13 @@ def test_queries_whose_lists_overflow_are_scanned_together(n, nq, metric):
     last = idx.last_bruteforce()
     assert last["scans"] == 1 and len(q[::2]) <= last["scanned"] < nq, last
     idx.close()
+
+
+@pytest.mark.parametrize("metric", [0, 1, 3])
+def test_one_large_query_does_not_send_the_others_to_the_scan(metric):
+    base, q = _normal(20000, 64, 11), _normal(150, 64, 12)
+    q[17] *= np.float32(1e12)
+    idx = DeviceIndex(vectors_only_graph(), base)
+    np.testing.assert_array_equal(idx.bruteforce(q, 10, metric), _words(base, q, 10, metric))
+    assert idx.last_bruteforce()["scanned"] <= 1
+    idx.close()
