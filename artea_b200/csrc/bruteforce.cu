@@ -118,8 +118,15 @@ struct BfArgs {
     uint32_t* __restrict__ part_n;         // nq x segments counts
 };
 
+// CTAs an SM: three leave 168 registers a thread, which the L2 metrics use without
+// spills; without the bound they took 180 and ran two (1,000 queries of 1M x 128:
+// 34.7 -> 37.0 ms). Dot (188) and cosine (238) would spill.
+constexpr int scan_min_blocks(int metric) {
+    return metric == ARTEA_GPU_EUCLIDEAN_SQR || metric == ARTEA_GPU_EUCLIDEAN ? 3 : 2;
+}
+
 template <int kMetric>
-__global__ void __launch_bounds__(kBfThreads) bf_scan_kernel(BfArgs a) {
+__global__ void __launch_bounds__(kBfThreads, scan_min_blocks(kMetric)) bf_scan_kernel(BfArgs a) {
     extern __shared__ __align__(16) unsigned char bf_smem[];
     uint64_t* lists = reinterpret_cast<uint64_t*>(bf_smem);                       // kBfQueries x list_cap
     float* qs = reinterpret_cast<float*>(lists + static_cast<size_t>(kBfQueries) * a.list_cap);  // kBfQueries x dim
