@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) bf_filter_kernel(const __grid_con
         const bool collect = a.limit != nullptr;
         const float beta = a.sign / pow2_scale(sqrtf(__uint_as_float(a.xs->max_sq))) * (valid ? a.qinfo[q].z : 0.0f);
         const f32x2 beta2 = pack2(beta, beta);
-        const float limit = collect && valid ? a.limit[q] : -INFINITY;
+        float limit = collect && valid ? a.limit[q] : -INFINITY;
         float m[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) m[i] = INFINITY;
@@ -420,6 +420,10 @@ __global__ void __launch_bounds__(kThreads, 1) bf_filter_kernel(const __grid_con
                     if (c >= kHitBuffer / 2u) {
                         filter_flush(a, hits, min(c, kHitBuffer));
                         if (lane == 0) hit_count[e] = 0;
+                        // A query whose list is full already goes to the scan: the rest
+                        // of its rows would be appended in vain (1M x 128 equal rows,
+                        // 1,000 queries, filter and scan: 49.0 -> 34.9 ms).
+                        if (valid && *reinterpret_cast<volatile uint32_t*>(a.count + q) > kListCap) limit = -INFINITY;
                         __syncwarp();
                     }
                 }

@@ -151,6 +151,19 @@ def test_queries_whose_lists_overflow_are_scanned_together(n, nq, metric):
     idx.close()
 
 
+@pytest.mark.parametrize("metric", [0, 2, 3])
+@pytest.mark.parametrize("nq", [4, 130])
+def test_every_list_overflows(nq, metric):
+    """All rows but 100 equal: a list is full after a few tiles, and the rest of them is not listed."""
+    base, q = np.tile(_normal(1, 48, 13), (70000, 1)), _normal(nq, 48, 14)
+    base[30000:30100] = _normal(100, 48, 15)
+    q[2] = base[30050]
+    idx = DeviceIndex(vectors_only_graph(), base)
+    np.testing.assert_array_equal(idx.bruteforce(q, 20, metric), _words(base, q, 20, metric))
+    assert idx.last_bruteforce()["scans"] == 1 and idx.last_bruteforce()["scanned"] >= nq - 1
+    idx.close()
+
+
 @pytest.mark.parametrize("metric", [0, 1, 3])
 def test_one_large_query_does_not_send_the_others_to_the_scan(metric):
     base, q = _normal(20000, 64, 11), _normal(150, 64, 12)
