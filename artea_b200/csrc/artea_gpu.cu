@@ -746,17 +746,20 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
     const bool pipe_open = a.l0_pipe && r->want_pipeline == 0;
     const bool fixed_pf = r->want_prefetch != 0 || !a.l0_pipe;
     const uint32_t pf_fixed = r->want_prefetch == 16 ? 1u : 0u;
+    const uint32_t slack_fixed = (r->want_slack == 0 || r->want_slack == kNoHash) ? 0u : r->want_slack;
+    // A team of two row warps exists for fixed-stride rows only.
+    const bool team2 = r->want_wpq == 2 && r->want_warps == 2 && a.l0_pipe;
     if (r->want_wpq > 1 && r->want_vh_bits) {
-        t.team = r->want_wpq == 4 ? 8u : 4u;
+        t.team = r->want_wpq == 4 ? 8u : (team2 ? 2u : 4u);
         t.warps = 1;
         t.vh_bits = hash_bits_of(r->want_vh_bits);
         t.regs = 2;
         t.stage = 0;
         t.pf = 0;
         t.pipe = 0;
+        t.slack = slack_fixed;
         return t;
     }
-    const uint32_t slack_fixed = (r->want_slack == 0 || r->want_slack == kNoHash) ? 0u : r->want_slack;
     if (r->want_wpq <= 1 && r->want_warps && r->want_vh_bits && r->want_regs && r->want_stage && fixed_pf) {
         t.warps = r->want_warps;
         t.vh_bits = hash_bits_of(r->want_vh_bits);
@@ -872,6 +875,7 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
     if (r->want_wpq == 1 || r->want_warps || r->want_regs || r->want_stage || r->want_prefetch ||
         r->want_pipeline == 1)
         team_choices.clear();   // those options describe the one-warp kernels
+    if (team2) team_choices = {2};
     for (uint32_t slack : slack_choices)
         for (uint32_t g : team_choices)
             for (uint32_t b : bit_choices) {
@@ -1364,7 +1368,7 @@ int artea_gpu_router_tuning(const artea_gpu_router* r, uint32_t* warps_per_cta, 
                             uint32_t* register_budget, uint32_t* stage_rows) {
     if (!r || !warps_per_cta || !visited_hash_bits || !register_budget || !stage_rows)
         return fail(ARTEA_GPU_EINVAL, "null argument");
-    *warps_per_cta = r->last.warps;
+    *warps_per_cta = r->last.team ? r->last.team : r->last.warps;
     *visited_hash_bits = r->last.vh_bits;
     *register_budget = regs_budget(r->last.regs);
     *stage_rows = r->last.stage;

@@ -179,7 +179,8 @@ typedef struct artea_gpu_router_opts {
                                    small team (2 or 4 warps reading rows and one
                                    keeping the queue) or a large one (8 and
                                    one), for batches that leave the GPU idle
-                                   and large dims; 0 = autotuned */
+                                   and large dims; 0 = autotuned. With 2,
+                                   warps_per_cta 2 takes the team of two */
     uint32_t queue_slack;       /* persistent kernels' queue layout:
                                    0xFFFFFFFF = 2L entries per search (room for
                                    every tie of lb the reference keeps);

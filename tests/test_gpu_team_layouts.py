@@ -1,0 +1,75 @@
+"""The options that pin a team's layout: the compact queue with its rerun, and
+the team of two row warps."""
+import numpy as np
+import pytest
+
+from artea_b200.graph import CompactHierarchicalGraph
+from artea_b200.router import DeviceIndex, GpuRouter
+from oracle import oracle as orc
+from test_gpu_team_search import _data, _graph
+
+pytestmark = pytest.mark.gpu
+
+NONE = 0xFFFFFFFF
+
+
+@pytest.fixture(scope="module", params=[(16, 64), (128, 40), (960, 33)], ids=lambda p: f"dim{p[0]}-deg{p[1]}")
+def case(request):
+    dim, deg = request.param
+    base = _data(1500, dim, dim)
+    g = _graph(base, deg, dim)
+    idx = DeviceIndex(g, base)
+    yield g, base, _data(70, dim, dim + 1), idx
+    idx.close()
+
+
+@pytest.mark.parametrize("wpq,row_warps", [(2, 2), (2, 4), (4, 8)])
+@pytest.mark.parametrize("bits,slack", [(6, 1), (9, 64), (NONE, 1)])
+def test_compact_queues(case, wpq, row_warps, bits, slack):
+    g, base, q, idx = case
+    ref, st = orc.batch_query(g, base, q, 40, 150, metric=0, stats=True)
+    r = GpuRouter(idx, 0, 40, 150, warps_per_query=wpq, warps_per_cta=2 if row_warps == 2 else 0,
+                  visited_hash_bits=bits, queue_slack=slack, schedule="persistent")
+    for _ in range(2):   # the visited set is left clear, by abandoned searches too
+        out, got = r.batch_query(q, stats=True)
+        np.testing.assert_array_equal(out, ref)
+        np.testing.assert_array_equal(got[:, :7], st[:, :7])
+        t = r.tuning()
+        assert (t["warps_per_query"], t["warps_per_cta"], t["queue_slack"]) == (wpq, row_warps, slack)
+        if slack == 1 and base.shape[1] == 16:   # distances tie often: some lose a live entry
+            assert r.last_reruns() > 0
+    r.close()
+
+
+@pytest.mark.parametrize("metric,mode", [(0, "fast"), (1, "exact"), (2, "exact"), (3, "exact")])
+@pytest.mark.parametrize("queue", [1, 32, 33, 300])
+def test_team_of_two_row_warps(case, queue, metric, mode):
+    g, base, q, idx = case
+    kw = dict(mode=mode, visited_hash_bits=8, schedule="persistent")
+    topk = min(queue, 50)
+    one = GpuRouter(idx, metric, topk, queue, warps_per_query=1, **kw)
+    ref, st = one.batch_query(q, stats=True)
+    one.close()
+    if mode == "exact":
+        np.testing.assert_array_equal(ref, orc.batch_query(g, base, q, topk, queue, metric=metric))
+    r = GpuRouter(idx, metric, topk, queue, warps_per_query=2, warps_per_cta=2, **kw)
+    out, got = r.batch_query(q, stats=True)
+    assert r.tuning()["warps_per_cta"] == 2
+    np.testing.assert_array_equal(out, ref)
+    np.testing.assert_array_equal(got[:, :7], st[:, :7])
+    np.testing.assert_array_equal(r.batch_query(q[:1]), ref[:1])
+    r.close()
+
+
+def test_a_pinned_team_of_two_without_fixed_stride_rows(case):
+    """A row with a repeated id has no fixed-stride copy: the team of four splits its distances."""
+    _, base, q, _ = case
+    n = 300
+    rows = [[[(v + 1 + j) % n for j in range(20)] + ([(v + 1) % n] if v % 7 == 0 else [])] for v in range(n)]
+    g = CompactHierarchicalGraph.from_rows(n, np.zeros(n, int), rows, 0, bl_max_nbr_size=64)
+    idx = DeviceIndex(g, base[:n])
+    r = GpuRouter(idx, 0, 10, 30, warps_per_query=2, warps_per_cta=2, visited_hash_bits=8, schedule="persistent")
+    np.testing.assert_array_equal(r.batch_query(q), orc.batch_query(g, base[:n], q, 10, 30, metric=0))
+    assert r.tuning()["warps_per_cta"] == 4
+    r.close()
+    idx.close()
