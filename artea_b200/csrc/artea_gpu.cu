@@ -758,6 +758,11 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
         t.pf = 0;
         t.pipe = 0;
         t.slack = slack_fixed;
+        // What does not fit beside a long queue is left out: a slack above the
+        // queue's own size, then the team's control block and so the team.
+        LaunchShape s;
+        if (t.slack && persistent_shape(r, t, &s) != ARTEA_GPU_OK) t.slack = 0;
+        if (persistent_shape(r, t, &s) != ARTEA_GPU_OK) t.team = 0;
         return t;
     }
     if (r->want_wpq <= 1 && r->want_warps && r->want_vh_bits && r->want_regs && r->want_stage && fixed_pf) {
@@ -913,6 +918,11 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
             }
     }
     for (auto& e : ev) cudaEventDestroy(e);
+    if (r->want_wpq > 1 && !r->want_warps && best_ms > 1e29f) {   // no team fits beside the queue
+        best.warps = 1;
+        best.regs = 2;
+        best.pipe = 0;
+    }
     r->tuned[key] = best;
     if (shared && best_ms < 1e29f) tuning_file_store(path, fkey, best);
     return best;

@@ -180,7 +180,9 @@ typedef struct artea_gpu_router_opts {
                                    keeping the queue) or a large one (8 and
                                    one), for batches that leave the GPU idle
                                    and large dims; 0 = autotuned. With 2,
-                                   warps_per_cta 2 takes the team of two */
+                                   warps_per_cta 2 takes the team of two.
+                                   A queue that leaves no room for a team is
+                                   searched by one warp */
     uint32_t queue_slack;       /* persistent kernels' queue layout:
                                    0xFFFFFFFF = 2L entries per search (room for
                                    every tie of lb the reference keeps);

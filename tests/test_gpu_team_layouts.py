@@ -1,5 +1,5 @@
-"""The options that pin a team's layout: the compact queue with its rerun, and
-the team of two row warps."""
+"""The options that pin a team's layout: the compact queue with its rerun, the
+team of two row warps, and queues that leave no room for a team's control block."""
 import numpy as np
 import pytest
 
@@ -71,5 +71,22 @@ def test_a_pinned_team_of_two_without_fixed_stride_rows(case):
     r = GpuRouter(idx, 0, 10, 30, warps_per_query=2, warps_per_cta=2, visited_hash_bits=8, schedule="persistent")
     np.testing.assert_array_equal(r.batch_query(q), orc.batch_query(g, base[:n], q, 10, 30, metric=0))
     assert r.tuning()["warps_per_cta"] == 4
+    r.close()
+    idx.close()
+
+
+@pytest.mark.parametrize("wpq", [2, 4])
+@pytest.mark.parametrize("bits", [0, NONE])
+@pytest.mark.parametrize("queue", [14400, 14454])
+def test_queue_that_leaves_no_room_for_a_team(wpq, bits, queue):
+    """Dim 16, no table: a search takes 16 queue + 1,152 bytes of 227 KB, a team 816 more."""
+    base = _data(1500, 16, 16)
+    g = _graph(base, 20, 7)
+    idx = DeviceIndex(g, base)
+    q = _data(9, 16, 8)
+    r = GpuRouter(idx, 0, 40, queue, warps_per_query=wpq, visited_hash_bits=bits, queue_slack=NONE,
+                  schedule="persistent")
+    np.testing.assert_array_equal(r.batch_query(q), orc.batch_query(g, base, q, 40, queue, metric=0))
+    assert r.tuning()["warps_per_query"] == (wpq if queue == 14400 else 1)
     r.close()
     idx.close()
