@@ -1035,6 +1035,21 @@ int index_begin(uint32_t num_vertices, const float* vectors, uint32_t num_vector
     return ARTEA_GPU_OK;
 }
 
+// A copy is made only where it leaves the visited sets of 32 searches an SM (the
+// most that a launch has in flight) and 1 GB for workspaces and batches: a program
+// that filled its device with vectors had these left for its routers.
+bool room_for_copy(const artea_gpu_index* ix, size_t bytes) {
+    size_t free_bytes = 0, total = 0;
+    int sms = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ix->device) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const size_t search = (static_cast<size_t>(ix->n) + 127) / 128 * 16 + 4u * std::min<size_t>(ix->n, 32768);
+    return free_bytes >= bytes + 32u * static_cast<size_t>(sms) * search + (size_t{1} << 30);
+}
+
 int index_finish_l0(artea_gpu_index* ix, const uint32_t* vertex_info, const uint64_t* const* group_offsets) {
     // Level-0 row descriptors (start | length << 40), one load per expansion.
     if (ix->n_nbrs >= (1ull << kRowLenShift) || ix->bl >= (1u << 24))
@@ -1069,7 +1084,7 @@ int index_finish_l0(artea_gpu_index* ix, const uint32_t* vertex_info, const uint
         // The fixed-stride copy of the level-0 rows (DeviceGraph::l0pad). It is
         // only an access path: without the memory for it the CSR rows serve.
         const size_t ids = static_cast<size_t>(ix->n) * kPadRow;
-        if (dev_alloc(&ix->d_l0pad, ids) == ARTEA_GPU_OK) {
+        if (room_for_copy(ix, sizeof(uint32_t) * ids) && dev_alloc(&ix->d_l0pad, ids) == ARTEA_GPU_OK) {
             l0_pad_kernel<<<std::max(sms, 1) * 8, 256>>>(ix->d_l0row, ix->d_nbrs, ix->n, ix->d_l0pad);
             if (cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess)
                 return fail(ARTEA_GPU_ECUDA, "level-0 rows failed");
@@ -1167,7 +1182,20 @@ int artea_gpu_index_destroy(artea_gpu_index* ix) {
 
 int artea_gpu_index_bytes(const artea_gpu_index* ix, uint64_t* bytes) {
     if (!ix || !bytes) return fail(ARTEA_GPU_EINVAL, "null argument");
-    *bytes = ix->bytes;
+    *bytes = ix->bytes + bf_rows_bytes(ix);
+    return ARTEA_GPU_OK;
+}
+
+int artea_gpu_index_lean(artea_gpu_index* ix) {
+    if (!ix) return fail(ARTEA_GPU_EINVAL, "null argument");
+    if (ix->routers.load()) return fail(ARTEA_GPU_EINVAL, "routers are alive on this index");
+    DeviceGuard guard(ix->device);
+    ix->lean = true;
+    if (ix->d_l0pad) {
+        dev_free(ix->d_l0pad);
+        ix->bytes -= sizeof(uint32_t) * static_cast<size_t>(ix->n) * kPadRow;
+    }
+    bf_drop_rows(ix);
     return ARTEA_GPU_OK;
 }
 
@@ -1208,6 +1236,7 @@ int artea_gpu_router_create(artea_gpu_index* ix, uint32_t topk, uint32_t queue, 
     DeviceGuard guard(ix->device);
     auto* r = new artea_gpu_router();
     r->idx = ix;
+    ++ix->routers;
     r->topk = topk;
     r->queue = queue;
     r->max_queue = std::max(o.max_queue ? o.max_queue : queue, queue);
@@ -1250,6 +1279,7 @@ int artea_gpu_router_destroy(artea_gpu_router* r) {
     if (!r) return ARTEA_GPU_OK;
     DeviceGuard guard(r->idx->device);
     if (r->stream) cudaStreamSynchronize(r->stream);
+    --r->idx->routers;
     clear_graphs(r);
     dev_free(r->d_vis_bits);
     dev_free(r->d_vis_list);

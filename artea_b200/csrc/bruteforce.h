@@ -31,7 +31,7 @@ struct BfStats {
 struct BfCache {
     int device = 0;
     std::mutex mu;                  // rows
-    bool norms_ready = false, rows_ready = false, rows_failed = false;
+    bool norms_ready = false, rows_ready = false;
     BfStats norms = {};             // host copy
     BfStats* d_norms = nullptr;
     __half* d_rows = nullptr;
@@ -64,6 +64,8 @@ struct BfWork {
 
 // Whether the index holds its rounded rows already.
 bool bf_rows_ready(const artea_gpu_index* ix);
+uint64_t bf_rows_bytes(const artea_gpu_index* ix);   // 0 without them
+void bf_drop_rows(const artea_gpu_index* ix);        // no call is running on the index
 
 // Ranks rows [0, n_rows) (or those of d_subset) for nq queries into d_out, and waits.
 // *used false: nothing was written (the filter does not apply). redo: queries left

@@ -999,6 +999,11 @@ namespace {
 
 size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
+// The index's rows in FP16, k_pad elements each.
+size_t rounded_bytes(const artea_gpu_index* ix) {
+    return static_cast<size_t>(ix->nvecs) * ((ix->dim + kChunkK - 1) / kChunkK * kChunkK) * sizeof(__half);
+}
+
 // With want_rows the index's rounded rows, made once; false where the filter cannot
 // be used (norms outside the bounds' range, no memory).
 bool bf_prepare(const artea_gpu_index* ix, bool want_rows, int sms, cudaStream_t st) {
@@ -1010,17 +1015,15 @@ bool bf_prepare(const artea_gpu_index* ix, bool want_rows, int sms, cudaStream_t
     std::memcpy(&mn, &c->norms.min_sq, 4);
     if (c->norms.bad || !(mx >= 1.0e-18f) || !(mx <= 1.0e18f) || !(mn >= 1.0e-18f)) return false;
     if (want_rows && !c->rows_ready) {
-        if (c->rows_failed) return false;
+        // Without the memory the call goes to the scan; a later one asks again.
         const uint32_t k_pad = (ix->dim + kChunkK - 1) / kChunkK * kChunkK;
-        if (dev_alloc(&c->d_rows, static_cast<size_t>(ix->nvecs) * k_pad) != ARTEA_GPU_OK) {
-            c->rows_failed = true;
+        if (ix->lean || !room_for_copy(ix, rounded_bytes(ix)) ||
+            dev_alloc(&c->d_rows, static_cast<size_t>(ix->nvecs) * k_pad) != ARTEA_GPU_OK)
             return false;
-        }
         bf_round_kernel<<<sms * 8, 256, 0, st>>>(ix->d_vecs, nullptr, ix->d_xsq, ix->nvecs, ix->dim, k_pad, c->d_norms,
                                                  c->d_rows, c->d_norms);
         if (cudaStreamSynchronize(st) != cudaSuccess) {   // other streams may use them next
             dev_free(c->d_rows);
-            c->rows_failed = true;
             return false;
         }
         c->rows_ready = true;
@@ -1033,6 +1036,14 @@ bool bf_prepare(const artea_gpu_index* ix, bool want_rows, int sms, cudaStream_t
 bool bf_rows_ready(const artea_gpu_index* ix) {
     std::lock_guard<std::mutex> lk(ix->bf->mu);
     return ix->bf->rows_ready;
+}
+
+uint64_t bf_rows_bytes(const artea_gpu_index* ix) { return bf_rows_ready(ix) ? rounded_bytes(ix) : 0u; }
+
+void bf_drop_rows(const artea_gpu_index* ix) {
+    std::lock_guard<std::mutex> lk(ix->bf->mu);
+    dev_free(ix->bf->d_rows);
+    ix->bf->rows_ready = false;
 }
 
 // Queries of a batch: bounds the workspace (16 query tiles keep every SM busy).

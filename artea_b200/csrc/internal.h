@@ -2,6 +2,7 @@
 // structure, error macro, device guard and device allocation helpers.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 
@@ -41,6 +42,8 @@ struct artea_gpu_index {
     uint64_t n_nbrs = 0;      // entries of d_nbrs in use
     uint64_t bytes = 0;
     artea_gpu::BfCache* bf = nullptr;   // brute force: rounded rows, workspace (bruteforce_tc.cu)
+    bool lean = false;                  // no copies beside the vectors and the CSR (artea_gpu_index_lean)
+    std::atomic<uint32_t> routers{0};   // alive on it: their captured launches hold its addresses
 };
 
 namespace artea_gpu {
@@ -86,5 +89,8 @@ int index_begin(uint32_t num_vertices, const float* vectors, uint32_t num_vector
 // group_offsets_host[h] on the host): the level-0 row descriptors and the
 // row-repeat check.
 int index_finish_l0(artea_gpu_index* ix, const uint32_t* vertex_info, const uint64_t* const* group_offsets_host);
+// Whether the device has room for a copy of so many bytes that only makes the
+// index's calls faster, beside what its calls need.
+bool room_for_copy(const artea_gpu_index* ix, size_t bytes);
 
 }  // namespace artea_gpu

@@ -116,6 +116,11 @@ class DeviceIndex:
         nat.check(nat.lib().artea_gpu_index_bytes(self.handle, ctypes.byref(b)))
         return int(b.value)
 
+    def lean(self) -> None:
+        """Give back the copies that only make calls faster, and make none any more
+        (artea_gpu_index_lean); before the first router."""
+        nat.check(nat.lib().artea_gpu_index_lean(self.handle))
+
     def bruteforce(self, queries: np.ndarray, topk: int, metric, subset: Optional[np.ndarray] = None) -> np.ndarray:
         """Exact brute-force top-k over this index's vectors (artea_gpu_bruteforce):
         (nq, topk) CandidateEntry words, ascending, CandidateEntry() padding."""

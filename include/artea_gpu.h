@@ -231,10 +231,15 @@ int artea_gpu_index_create_from_hgra(const char* path, const float* vectors, uin
 int artea_gpu_index_download(const artea_gpu_index* index, uint32_t* vertex_info, uint64_t* offsets,
                              uint32_t* neighbor_ids);
 int artea_gpu_index_destroy(artea_gpu_index* index);
-/* Device bytes held by the index (vectors, their x.x row norms, CSR, and the
- * level-0 rows at a fixed stride of 64 ids where every row holds at most 64
- * distinct ones). */
+/* Device bytes held by the index: vectors, their x.x row norms, CSR, the level-0
+ * rows at a fixed stride of 64 ids where every row holds at most 64 distinct ones,
+ * and the FP16 rows of brute force once a call made them. The last two are copies
+ * that only make calls faster, and are made only where they leave room for the
+ * visited sets of a full launch and 1 GB. */
 int artea_gpu_index_bytes(const artea_gpu_index* index, uint64_t* bytes);
+/* Gives both copies back and makes none on this index any more. Results stay the
+ * same. EINVAL while a router is alive on the index; no call may be running on it. */
+int artea_gpu_index_lean(artea_gpu_index* index);
 
 /* ---- Router ---- */
 /* topk / candidate_queue_size are the defaults used when a call passes no
