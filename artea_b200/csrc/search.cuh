@@ -412,7 +412,12 @@ __device__ void batch_distances(const DeviceGraph& g, const float* __restrict__ 
     const uint32_t dim = g.dim;
     const uint32_t nchunks = dim >> 4;
     const uint32_t sstride = dim + kStagePad;
-    if (kNarrow && !kStage && !kSplit) {   // level 0 of the benchmark's widths: 128 and 96
+    // Level 0, rows of 128 and 96 elements. The other widths up to 128 stay on the
+    // masked loop: the same code with their number of chunks in a register takes more
+    // of them, and the autotuner then leaves the 96-register kernels (1M rows, 10,000
+    // queries, queue 100: 16 elements 2.64 -> 3.02 ms, 64 3.15 -> 3.57, 112 3.51 ->
+    // 3.98, and 128 itself 2.82 -> 3.03; without the two widths' own code 128 3.75 ms).
+    if (kNarrow && !kStage && !kSplit) {
         if (nchunks == 8u) return narrow_distances<kMetric, kExact, kPre, 8>(g, q, qsq, cvid, cdist, cnt, pre);
         if (nchunks == 6u) return narrow_distances<kMetric, kExact, kPre, 6>(g, q, qsq, cvid, cdist, cnt, pre);
     }
