@@ -363,15 +363,22 @@ int scan(const artea_gpu_index* ix, int metric, const float* d_queries, uint32_t
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(fn), kBfThreads,
                                                            smem));
     const uint32_t tiles = (nq + kBfQueries - 1) / kBfQueries;
-    // Split the rows into segments until the grid covers the GPU twice over. A
-    // segment has at least 512 rows (4 rounds of its CTA) and 32 per result, since
-    // each hands k keys to the merge, which sorts them in shared memory: up to 4,096
-    // keys, or two segments an SM where k is large. (4,096 rows a segment left one
-    // query over 200k rows on 48 CTAs.)
-    const uint32_t want = 2u * static_cast<uint32_t>(std::max(per_sm, 1) * dev_sms);
-    uint32_t segments = std::max(1u, (want + tiles - 1) / tiles);
-    segments = std::min(segments, std::max(1u, n_rows / std::min(4096u, std::max(512u, 32u * topk))));
-    segments = std::min(segments, std::max(4096u / topk, 2u * static_cast<uint32_t>(dev_sms)));
+    // Rows are split into segments: one a CTA, whose lists are sorted at its end and
+    // merged (about 100 us of its time at 384 keys, whatever the segment's length).
+    // - Of 4,096 rows or more: until the grid covers the GPU twice over.
+    // - Of 512 rows (4 rounds of a CTA) and 32 per result or more: until there are two
+    //   CTAs an SM. (1,000 queries over 4,096 x 16 rows: 1, 2, 4 and 8 segments 222, 190,
+    //   309 and 430 us; one query over 200k rows was left on 48 CTAs by 4,096 rows each.)
+    // - With more CTAs than that: halves, where they save a quarter of the waves and are
+    //   well longer than the sort (cosine, 2 CTAs an SM, 2,500 queries: over 8,191 x 400
+    //   rows 2.79 -> 2.24 ms, over 4,096 x 96 rows 0.69 -> 0.75).
+    const uint32_t sms = static_cast<uint32_t>(dev_sms), slots = static_cast<uint32_t>(std::max(per_sm, 1)) * sms;
+    const uint32_t whole = std::min((2u * slots + tiles - 1) / tiles, n_rows / 4096u);
+    const uint32_t fill = std::min(2u * sms / tiles, n_rows / std::min(4096u, std::max(512u, 32u * topk)));
+    const bool halves = 2u * ((2u * tiles + slots - 1) / slots) <= 3u * ((tiles + slots - 1) / slots) &&
+                        static_cast<uint64_t>(n_rows / 2u) * ix->dim >= 1000000u;
+    uint32_t segments = std::max({1u, whole, fill, tiles > 2u * sms && halves ? 2u : 1u});
+    segments = std::min(segments, std::max(4096u / topk, 2u * sms));
     segments = std::min(segments, std::max(1u, kMergeKeys / topk));
     const uint32_t seg_len = (n_rows + segments - 1) / segments;
     segments = (n_rows + seg_len - 1) / seg_len;
