@@ -50,7 +50,8 @@ struct Tuning {
     uint32_t stage = 0;  // 0: rows read with vector loads; kStageRows: TMA-staged in shared memory
     uint32_t pf = 0;     // pipelined level-0 loop: 1 = the second pass's rows are prefetched into L2
     uint32_t pipe = 1;   // pipelined level-0 loop where the graph allows it (0: one expansion at a time)
-    uint32_t team = 0;   // row warps of the team kernel (2, 4 or 8; a CTA searches a query); 0: a warp per query
+    uint32_t team = 0;   // row warps of the team kernel (2, 4 or 8, without fixed-stride rows 1 or 3; a CTA
+                         // searches a query); 0: a warp per query
     uint32_t slack = 0;  // queue layout: 0 = 2L entries per search; > 0 = compact, max queue + slack
                          // entries, a query that could lose a live entry is rerun at 2L
 };
@@ -280,17 +281,21 @@ KernelFn pick_kernel_m(bool exact, bool persistent, uint32_t regs, bool stage, b
 }
 
 // Router option warps_per_query: 1 = a warp per query, 2 = a small team (2 or 4
-// row warps), 4 = a large one (8).
-uint32_t wpq_of(uint32_t team) { return team == 0 ? 1u : (team == 8 ? 4u : 2u); }
+// row warps; 1 without fixed-stride rows), 4 = a large one (8; 3).
+uint32_t wpq_of(uint32_t team) { return team == 0 ? 1u : (team == 8 || team == 3 ? 4u : 2u); }
 
-// pad: level 0 split over the team (graphs with fixed-stride rows); without it
-// the teams of 4 and 8 only split the distance batches.
+// pad: level 0 split over the team (graphs with fixed-stride rows). Without it the
+// warps only split the distance batches, the leader among them: 2 or 4 warps a CTA,
+// since more of them wait for the leader most of the time (100k x 128, 3,000
+// queries, queue 400: 4 warps 16.1 ms, 9 warps 22.5; 40k x 960 29.2 and 59.9 ms).
 template <int kMetric, bool kExact>
 KernelFn pick_team_e(uint32_t team, bool pad) {
     switch (team) {
+        case 1: return pad ? nullptr : search_team_kernel<kMetric, kExact, 1, false>;
         case 2: return pad ? search_team_kernel<kMetric, kExact, 2, true> : nullptr;
-        case 4: return pad ? search_team_kernel<kMetric, kExact, 4, true> : search_team_kernel<kMetric, kExact, 4, false>;
-        case 8: return pad ? search_team_kernel<kMetric, kExact, 8, true> : search_team_kernel<kMetric, kExact, 8, false>;
+        case 3: return pad ? nullptr : search_team_kernel<kMetric, kExact, 3, false>;
+        case 4: return pad ? search_team_kernel<kMetric, kExact, 4, true> : nullptr;
+        case 8: return pad ? search_team_kernel<kMetric, kExact, 8, true> : nullptr;
         default: return nullptr;
     }
 }
@@ -701,7 +706,7 @@ bool tuning_file_load(const std::string& path, const std::string& fkey, Tuning* 
         unsigned w, b, rg, st, pf, pp, q, sl;
         if (std::sscanf(line, "%599s %u %u %u %u %u %u %u %u", k, &w, &b, &rg, &st, &pf, &pp, &q, &sl) == 9 &&
             fkey == k && rg <= 3 && (st == 0 || st == kStageRows) && pf <= 1 && pp <= 1 && w >= 1 && w <= 8 &&
-            b <= 12 && (q == 0 || q == 2 || q == 4 || q == 8) && sl <= 4096) {
+            b <= 12 && (q <= 4 || q == 8) && sl <= 4096) {
             t->team = q;
             t->slack = sl;
             t->warps = w;
@@ -750,7 +755,7 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
     // A team of two row warps exists for fixed-stride rows only.
     const bool team2 = r->want_wpq == 2 && r->want_warps == 2 && a.l0_pipe;
     if (r->want_wpq > 1 && r->want_vh_bits) {
-        t.team = r->want_wpq == 4 ? 8u : (team2 ? 2u : 4u);
+        t.team = !a.l0_pipe ? r->want_wpq - 1u : (r->want_wpq == 4 ? 8u : (team2 ? 2u : 4u));
         t.warps = 1;
         t.vh_bits = hash_bits_of(r->want_vh_bits);
         t.regs = 2;
@@ -876,7 +881,7 @@ Tuning tuned(artea_gpu_router* r, const SearchArgs& a, cudaStream_t st) {
                         time_candidate(c);
                     }
     // 1b. warps per query: the team kernel at every team and table size.
-    std::vector<uint32_t> team_choices = {2, 4, 8};
+    std::vector<uint32_t> team_choices = a.l0_pipe ? std::vector<uint32_t>{2, 4, 8} : std::vector<uint32_t>{1, 3};
     if (r->want_wpq == 1 || r->want_warps || r->want_regs || r->want_stage || r->want_prefetch ||
         r->want_pipeline == 1)
         team_choices.clear();   // those options describe the one-warp kernels

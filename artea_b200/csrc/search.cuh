@@ -2016,10 +2016,12 @@ __device__ void team_rows(const SearchArgs& a, const WarpSmem& sm, int warp) {
         const uint32_t cmd = ctl->cmd;
         const float qsq = ctl->qsq;
         if (cmd == kCmdQuit) break;
-        if (kPad && cmd == kCmdLevel0) {
-            if ((a.g.dim >> 4) <= kBlock) l0_team_rows<kMetric, kExact, kG, false>(a, sm, vs, warp - 1, qsq);
-            else l0_team_rows<kMetric, kExact, kG, true>(a, sm, vs, warp - 1, qsq);
-            continue;
+        if constexpr (kPad) {
+            if (cmd == kCmdLevel0) {
+                if ((a.g.dim >> 4) <= kBlock) l0_team_rows<kMetric, kExact, kG, false>(a, sm, vs, warp - 1, qsq);
+                else l0_team_rows<kMetric, kExact, kG, true>(a, sm, vs, warp - 1, qsq);
+                continue;
+            }
         }
         batch_distances<kMetric, kExact, false, false, true>(a.g, sm.q, qsq, ctl->cvid, ctl->cdist, ctl->cnt, st,
                                                             a.error, nullptr, static_cast<uint32_t>(warp), kG + 1);
@@ -2510,7 +2512,7 @@ __global__ void __launch_bounds__(32, 24) search_rerun_kernel(SearchArgs a) {
 // time (queries from the shared counter, in a.order if set). Rows are read with
 // vector loads. Launch bounds leave at least 96 registers a thread: the row
 // warps hold the expected expansion's first rows in registers.
-constexpr int team_min_blocks(int g) { return g == 2 ? 6 : (g == 4 ? 4 : 2); }
+constexpr int team_min_blocks(int g) { return g == 1 ? 10 : (g == 2 ? 6 : (g == 3 ? 5 : (g == 4 ? 4 : 2))); }
 
 // kPad: level 0 split over the team (fixed-stride rows); else one expansion at a
 // time by the leader, its distance batches split over the warps.

@@ -181,6 +181,8 @@ typedef struct artea_gpu_router_opts {
                                    one), for batches that leave the GPU idle
                                    and large dims; 0 = autotuned. With 2,
                                    warps_per_cta 2 takes the team of two.
+                                   Where level 0 has no fixed-stride rows: 2 or
+                                   4 warps that split the distances.
                                    A queue that leaves no room for a team is
                                    searched by one warp */
     uint32_t queue_slack;       /* persistent kernels' queue layout:

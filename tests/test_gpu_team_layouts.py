@@ -61,16 +61,23 @@ def test_team_of_two_row_warps(case, queue, metric, mode):
     r.close()
 
 
-def test_a_pinned_team_of_two_without_fixed_stride_rows(case):
-    """A row with a repeated id has no fixed-stride copy: the team of four splits its distances."""
+@pytest.mark.parametrize("wpq,slack", [(2, NONE), (4, NONE), (2, 1), (4, 64)])
+@pytest.mark.parametrize("bits", [0, 8])
+def test_teams_without_fixed_stride_rows(case, wpq, slack, bits):
+    """A row with a repeated id has no fixed-stride copy: 2 or 4 warps split the distances, the leader among them."""
     _, base, q, _ = case
     n = 300
     rows = [[[(v + 1 + j) % n for j in range(20)] + ([(v + 1) % n] if v % 7 == 0 else [])] for v in range(n)]
     g = CompactHierarchicalGraph.from_rows(n, np.zeros(n, int), rows, 0, bl_max_nbr_size=64)
     idx = DeviceIndex(g, base[:n])
-    r = GpuRouter(idx, 0, 10, 30, warps_per_query=2, warps_per_cta=2, visited_hash_bits=8, schedule="persistent")
-    np.testing.assert_array_equal(r.batch_query(q), orc.batch_query(g, base[:n], q, 10, 30, metric=0))
-    assert r.tuning()["warps_per_cta"] == 4
+    ref, st = orc.batch_query(g, base[:n], q, 10, 30, metric=0, stats=True)
+    r = GpuRouter(idx, 0, 10, 30, warps_per_query=wpq, visited_hash_bits=bits, queue_slack=slack,
+                  schedule="persistent")
+    out, got = r.batch_query(q, stats=True)
+    np.testing.assert_array_equal(out, ref)
+    np.testing.assert_array_equal(got[:, :7], st[:, :7])
+    t = r.tuning()
+    assert (t["warps_per_query"], t["warps_per_cta"]) == (wpq, wpq - 1)
     r.close()
     idx.close()
 
