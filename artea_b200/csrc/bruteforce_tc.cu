@@ -23,6 +23,9 @@
 // the rows' largest R), the accumulation in the tensor core (2^-19 of |q||x| per
 // 16 products, 32 times the unit of its FP32 accumulator), the FP32 chain of the
 // distance itself, and the rounding of sqrt (distances that are equal after it).
+// The accumulation's share is a margin and no documented property: against 64 bits on
+// the same FP16 operands it took at most 5 % of it, at 64 to 2,048 elements of normal,
+// one-signed, cancelling and widely spread values.
 // A query whose list does not fit, or an index or query whose norms leave the
 // range in which these bounds hold, goes to the FP32 scan: rows that are not
 // finite or whose nonzero norms leave [10^-9, 10^9], queries above 10^15, and for

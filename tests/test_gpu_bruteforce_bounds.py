@@ -172,3 +172,22 @@ def test_one_large_query_does_not_send_the_others_to_the_scan(metric):
     np.testing.assert_array_equal(idx.bruteforce(q, 10, metric), _words(base, q, 10, metric))
     assert idx.last_bruteforce()["scanned"] <= 1
     idx.close()
+
+
+@pytest.mark.parametrize("metric", [0, 2, 3])
+@pytest.mark.parametrize("nq", [3, 40])
+def test_subset_with_repeated_ids(nq, metric):
+    """An id comes as often as the subset holds it; the words are in order of (distance, id)."""
+    rng = np.random.default_rng(16)
+    base, q = _normal(12000, 96, 17), _normal(nq, 96, 18)
+    sub = rng.permutation(12000)[:6000].astype(np.uint32)
+    sub = rng.permutation(np.concatenate([sub, sub[:3000], sub[:500], sub[:100]]))
+    rows = np.sort(sub)   # the oracle's ties: by position
+    ids, d = orc.bruteforce(base[rows], q, 60, metric=metric)
+    want = (d.view(np.uint32).astype(np.uint64) << np.uint64(32)) | rows[ids].astype(np.uint64)
+    assert (want[:, 1:] == want[:, :-1]).any()
+    idx = DeviceIndex(vectors_only_graph(), base)
+    np.testing.assert_array_equal(idx.bruteforce(q, 60, metric, sub), want)
+    idx.bruteforce(q, 60, metric)
+    np.testing.assert_array_equal(idx.bruteforce(q, 60, metric, sub), want)
+    idx.close()
