@@ -31,6 +31,7 @@ whole index and answers its own batch; times are the max over ranks.
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import os
 import statistics
@@ -203,11 +204,18 @@ def measured_peaks() -> dict:
     return {"hbm_gbs": 6650.0, "source": "fallback"}
 
 
+def search_source() -> str:
+    """The search kernels' source, as summaries name it: 12 digits of search.cuh's SHA-1."""
+    with open(os.path.join(ROOT, "artea_b200", "csrc", "search.cuh"), "rb") as f:
+        return hashlib.sha1(f.read()).hexdigest()[:12]
+
+
 def profile_traffic(workload: str, tuning: dict, alg_bytes: float, queue=None):
     """DRAM read+write bytes per launch of the timed kernel from the committed
     ncu summary of this workload (profiles/search_kernel_<workload>.md), and
     where the figure came from; (None, reason) unless the summary's
-    `captured_tuning:` line names the same kernel variant as the timed launch.
+    `captured_tuning:` line names the same kernel variant as the timed launch and its
+    `captured_source:` line the kernels' source (search_source()).
     The summary gives either `traffic_bytes_per_launch[_L<queue>]:` (a capture
     of this launch) or `dram_bytes_per_algorithmic_byte:` (a capture of a
     smaller case of the same kernel, scaled here by this launch's algorithmic
@@ -216,8 +224,10 @@ def profile_traffic(workload: str, tuning: dict, alg_bytes: float, queue=None):
     if not os.path.exists(p):
         return None, f"no ncu summary for {workload}"
     lines = [line.strip() for line in open(p)]
-    captured = None
+    captured, source = None, None
     for line in lines:
+        if line.startswith("captured_source:"):
+            source = line.split(":", 1)[1].strip()
         if line.startswith("captured_tuning:"):
             try:
                 captured = json.loads(line.split(":", 1)[1])
@@ -225,6 +235,8 @@ def profile_traffic(workload: str, tuning: dict, alg_bytes: float, queue=None):
                 captured = None
     if not captured or any(tuning.get(k) != v for k, v in captured.items()):
         return None, f"the ncu summary's kernel variant {captured} is not the timed one"
+    if source != search_source():
+        return None, "the ncu summary was captured with other sources of the search kernels"
 
     def number(key):
         for line in lines:
@@ -884,7 +896,11 @@ def main() -> None:
     args.warmup = max(args.warmup, 3)
 
     if args.impl == "reference":
-        run_reference_arm(args)
+        try:
+            run_reference_arm(args)
+        except FileNotFoundError as e:   # no graph without the reference's builder
+            if os.environ.get("RANK", "0") == "0":
+                print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
         return
 
     import torch
