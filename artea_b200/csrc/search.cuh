@@ -819,7 +819,7 @@ __device__ __forceinline__ void visited_test_and_set2(Visited& vs, uint32_t v0, 
     if (vs.tbits) table_test_insert2(vs, v0, a0, v1, a1, &t0, &t1);
     // Both bitset tests are issued before either result is used: one DRAM latency
     // an expansion in place of two (1M x 128, 10,000 queries, 4 KB table: queue 400
-    // 11.4 -> 10.6 ms, queue 100 3.16 -> 3.05 ms).
+    // 11.6 -> 10.6 ms, queue 100 3.22 -> 3.05 ms).
     const uint32_t mask0 = 1u << (v0 & 31), mask1 = 1u << (v1 & 31);
     uint32_t old0 = ~0u, old1 = ~0u;
     if (t0 == 2) old0 = atomicOr(vs.bits + (v0 >> 5), mask0);
