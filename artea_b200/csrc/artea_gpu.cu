@@ -663,8 +663,9 @@ int launch_graph(artea_gpu_router* r, SearchArgs a, bool persistent, const Tunin
 // Picks are kept per router and, for routers that fix none of these options, in a text file (ARTEA_TUNING_CACHE; default
 // $XDG_CACHE_HOME/artea_b200/tuning.txt, else ~/.cache/artea_b200/tuning.txt;
 // an empty ARTEA_TUNING_CACHE turns the file off) keyed by the GPU model, SM
-// count, this library's build, the metric, mode, graph size and the
-// combination above, so later processes skip the timing.
+// count, this library's build, the metric, mode, graph size, whether the index
+// has fixed-stride rows (other kernels, other picks) and the combination above,
+// so later processes skip the timing.
 const char* kBuildId = __DATE__ " " __TIME__;
 
 std::string tuning_cache_path() {
@@ -685,9 +686,9 @@ std::string tuning_file_key(const artea_gpu_router* r, uint64_t key) {
     if (cudaGetDeviceProperties(&prop, r->idx->device) == cudaSuccess) gpu = prop.name;
     else cudaGetLastError();
     char buf[512];
-    std::snprintf(buf, sizeof(buf), "%s|%d|%s|m%d|x%d|n%u|k%llx|cs%u|p%u|o%u", gpu.c_str(), r->num_sms, kBuildId,
-                  r->metric, r->mode, r->idx->n, static_cast<unsigned long long>(key), r->want_ctas_per_sm,
-                  r->want_pipeline, r->want_order);
+    std::snprintf(buf, sizeof(buf), "%s|%d|%s|m%d|x%d|n%u|f%d|k%llx|cs%u|p%u|o%u", gpu.c_str(), r->num_sms, kBuildId,
+                  r->metric, r->mode, r->idx->n, r->idx->d_l0pad ? 1 : 0, static_cast<unsigned long long>(key),
+                  r->want_ctas_per_sm, r->want_pipeline, r->want_order);
     std::string k(buf);
     for (char& c : k)
         if (c == ' ') c = '_';

@@ -86,3 +86,34 @@ def test_rounded_rows_are_made_once_there_is_room():
     np.testing.assert_array_equal(idx.bruteforce(q, 10, 0), scanned)
     assert idx.last_bruteforce()["scanned"] == 0 and idx.nbytes() == before + 1_000_000 * 128
     idx.close()
+
+
+def test_saved_picks_stay_with_the_rows_they_were_timed_with(tmp_path, monkeypatch):
+    """Teams of 2, 4 and 8 row warps exist for fixed-stride rows alone, teams of 1 and 3 without them alone;
+    two indexes that differ in nothing else share a tuning file."""
+    path = tmp_path / "tuning.txt"
+    monkeypatch.setenv("ARTEA_TUNING_CACHE", str(path))
+    base, q = _data(1500, 48, 4), _data(20, 48, 5)
+    g = _graph(base, 24, 6)
+    ref = orc.batch_query(g, base, q, 20, 60, metric=0)
+    whole, lean = DeviceIndex(g, base), DeviceIndex(g, base)
+    lean.lean()
+
+    def run(idx):
+        r = GpuRouter(idx, 0, 20, 60, schedule="persistent")
+        np.testing.assert_array_equal(r.batch_query(q), ref)
+        t = r.tuning()
+        r.close()
+        return t
+
+    for first, second, teams in ((whole, lean, (2, 4, 8)), (lean, whole, (1, 3))):
+        path.write_text("")
+        run(first)
+        key = path.read_text().split()[0]
+        for team in teams:
+            path.write_text(f"{key} 1 8 2 0 0 0 {team} 0\n")   # the pick: this team
+            assert run(first)["warps_per_cta"] == team
+            run(second)
+            assert len({line.split()[0] for line in path.read_text().splitlines()}) == 2
+    whole.close()
+    lean.close()
