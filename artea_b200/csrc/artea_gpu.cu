@@ -82,6 +82,8 @@ struct GraphKey {
 
 struct artea_gpu_router {
     artea_gpu_index* idx = nullptr;
+    int device = 0;                                  // the index's
+    std::shared_ptr<std::atomic<uint32_t>> counted;  // the index's count of its routers
     uint32_t topk = 0, queue = 0, max_queue = 0, cap = 0, max_batch = 0;
     int metric = 0, mode = 0, schedule = 0;
     uint32_t want_warps = 0, want_ctas_per_sm = 0, want_vh_bits = 0, want_regs = 0, want_stage = 0;
@@ -1194,7 +1196,7 @@ int artea_gpu_index_bytes(const artea_gpu_index* ix, uint64_t* bytes) {
 
 int artea_gpu_index_lean(artea_gpu_index* ix) {
     if (!ix) return fail(ARTEA_GPU_EINVAL, "null argument");
-    if (ix->routers.load()) return fail(ARTEA_GPU_EINVAL, "routers are alive on this index");
+    if (ix->routers->load()) return fail(ARTEA_GPU_EINVAL, "routers are alive on this index");
     DeviceGuard guard(ix->device);
     ix->lean = true;
     if (ix->d_l0pad) {
@@ -1242,7 +1244,9 @@ int artea_gpu_router_create(artea_gpu_index* ix, uint32_t topk, uint32_t queue, 
     DeviceGuard guard(ix->device);
     auto* r = new artea_gpu_router();
     r->idx = ix;
-    ++ix->routers;
+    r->device = ix->device;
+    r->counted = ix->routers;
+    ++*r->counted;
     r->topk = topk;
     r->queue = queue;
     r->max_queue = std::max(o.max_queue ? o.max_queue : queue, queue);
@@ -1283,9 +1287,9 @@ int artea_gpu_router_create(artea_gpu_index* ix, uint32_t topk, uint32_t queue, 
 
 int artea_gpu_router_destroy(artea_gpu_router* r) {
     if (!r) return ARTEA_GPU_OK;
-    DeviceGuard guard(r->idx->device);
+    DeviceGuard guard(r->device);   // (the index may be gone)
     if (r->stream) cudaStreamSynchronize(r->stream);
-    --r->idx->routers;
+    --*r->counted;
     clear_graphs(r);
     dev_free(r->d_vis_bits);
     dev_free(r->d_vis_list);

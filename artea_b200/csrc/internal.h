@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <memory>
 #include <string>
 
 #include <cuda_runtime.h>
@@ -43,7 +44,9 @@ struct artea_gpu_index {
     uint64_t bytes = 0;
     artea_gpu::BfCache* bf = nullptr;   // brute force: rounded rows, workspace (bruteforce_tc.cu)
     bool lean = false;                  // no copies beside the vectors and the CSR (artea_gpu_index_lean)
-    std::atomic<uint32_t> routers{0};   // alive on it: their captured launches hold its addresses
+    // Routers alive on it: their captured launches hold its addresses. Shared with them,
+    // since a router may be destroyed after its index.
+    std::shared_ptr<std::atomic<uint32_t>> routers = std::make_shared<std::atomic<uint32_t>>(0u);
 };
 
 namespace artea_gpu {

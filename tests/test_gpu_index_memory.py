@@ -117,3 +117,18 @@ def test_saved_picks_stay_with_the_rows_they_were_timed_with(tmp_path, monkeypat
             assert len({line.split()[0] for line in path.read_text().splitlines()}) == 2
     whole.close()
     lean.close()
+
+
+def test_a_router_closed_after_its_index_leaves_the_next_index_alone():
+    """The next index mostly takes the memory of the one destroyed before it; its count of routers stays 0."""
+    base = _data(300, 16, 1)
+    g = _graph(base, 24, 2)
+    for _ in range(8):
+        idx = DeviceIndex(g, base)
+        routers = [GpuRouter(idx, 0, 5, 20) for _ in range(3)]
+        idx.close()
+        following = DeviceIndex(g, base)
+        for r in routers:
+            r.close()
+        following.lean()   # refused while a router is alive on it
+        following.close()
